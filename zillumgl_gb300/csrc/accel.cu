@@ -1,6 +1,7 @@
 // accel.cu — MTBVH upload and the closest-hit / any-hit trace kernels, plus
 // the zgl_accel_* and zgl_trace_* entry points.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -9,6 +10,7 @@
 
 #include "accel.h"
 #include "traverse.cuh"
+#include "wide.cuh"
 #include "zgl_internal.h"
 
 namespace zgl {
@@ -97,6 +99,171 @@ trace_count_kernel(DeviceAccel a, const float* __restrict__ org, const float* __
     }
     visits[i] = v;
     tests[i] = t;
+}
+
+// Rays of a warp that the wide tree's loop leaves out, marked by `want`: the
+// rarer modes one per lane on the wide tree, the others (and those whose
+// stack ran out) on the face table, past kLaneBudget entries with the whole
+// warp.  Every lane calls.
+template <bool ANY>
+static __device__ __noinline__ void trace_rest(DeviceAccel a, const float* org, const float* dir, const float* tmax,
+                                               int64_t i, bool want, bool overflow, int32_t* hit_id, float* hit_t,
+                                               uint8_t* occ) {
+    const TraceRay r = lane_ray(org, dir, i, want);
+    float dist = ANY ? (want ? tmax[i] : 0.0f) : 1e8f;
+    int closest = -1;
+    bool done = !want;
+    if (want && !overflow && wide_covers(r)) {
+        const WideHit h = traverse_wide<ANY, true>(a, r, dist);
+        if (h.ok) {
+            closest = h.id;
+            dist = h.dist;
+            done = true;
+        }
+    }
+    if (!__all_sync(0xffffffffu, done)) {
+        int k = 0;
+        done = done || traverse_lane_m<ANY, false, 0>(a, r, dist, k, closest, kLaneBudget);
+        finish_long_rays<ANY>(a, r, dist, k, closest, done);
+    }
+    if (!want) return;
+    if (ANY) {
+        occ[i] = (uint8_t)(closest >= 0);
+    } else {
+        hit_id[i] = closest;
+        hit_t[i] = dist;
+    }
+}
+
+// The default schedule: closest or any hit of every ray on the wide tree.
+//
+// Divergence is what this loop fights.  Rays of one warp visit between a few
+// and 400 nodes (mean 31 on the 4M soup's bounce rays, 4 triangles); one ray
+// per thread to the end kept 5.5 lanes busy and ran at 740 Mrays/s.  So
+//  * the grid is one wave of resident warps, each taking every nwarps-th group
+//    of 32 rays; lanes without a ray are refilled from the sequence once
+//    kRefill of them are idle (no counter in memory, so launches on other
+//    streams and in graphs stay independent).  256 consecutive rays per warp
+//    instead: 1083 Mrays/s, one wave: 1268 (its tails come once a launch);
+//  * a lane that reaches a triangle sets it aside and goes on with the nodes
+//    behind it (a later, larger distance only adds nodes; triangles are still
+//    tested in order).  The warp turns to the waiting triangles when fewer
+//    than kInner lanes have a node left (8 to 24 measured, flat at 16 to 20).
+// 64-byte nodes in two 32-byte loads: with 128-byte nodes of full floats in
+// eight 16-byte loads the L1 was 70% busy (a gather takes a cycle a lane) and
+// the same loop ran at 760 Mrays/s.  48 registers (20 warps of 64 threads per
+// SM) hide more latency than 64 (1192) or 40 (1268 and slower when coherent).
+constexpr int kWideBlock = 64;
+constexpr int kWideBlocksPerSM = 20;
+constexpr int kInner = 16;
+constexpr int kRefill = 8;
+
+template <bool ANY>
+__global__ void __launch_bounds__(kWideBlock, kWideBlocksPerSM)
+trace_wide_kernel(DeviceAccel a, const float* __restrict__ org, const float* __restrict__ dir,
+                  const float* __restrict__ tmax, int64_t n, int group, int32_t* __restrict__ hit_id,
+                  float* __restrict__ hit_t, uint8_t* __restrict__ occ) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u;
+    // ray p of this warp's sequence is ray ((p / 32) * nwarps + warp) * 32 +
+    // p % 32; with fewer rays than that takes, the warp has `group` of them
+    const int64_t warp = blockIdx.x * (int64_t)(kWideBlock / 32) + (threadIdx.x >> 5);
+    const int64_t nwarps = gridDim.x * (int64_t)(kWideBlock / 32);
+    int64_t taken = 0;
+    bool more = warp * group < n;
+    int stack[kWideStack];
+    stack[0] = kWideDone;
+    int64_t ray = 0;
+    TraceRay r;
+    const WidePad none{};
+    float dist = 0.0f;
+    int closest = -1, sp = 1, cur = kWideDone, leaf = 0;
+    bool live = false;
+    for (;;) {
+        // refill the lanes without a ray
+        const unsigned idle = __ballot_sync(full, !live);
+        if (idle == full && !more) break;
+        if (more && __popc(idle) >= kRefill) {
+            const int64_t p = taken + __popc(idle & lt);
+            int64_t mine;
+            if (group == 32) {
+                mine = ((p >> 5) * nwarps + warp) * 32 + (p & 31);
+                taken += __popc(idle);
+                more = ((taken >> 5) * nwarps + warp) * 32 + (taken & 31) < n;
+            } else {
+                mine = p < group ? warp * group + p : n;
+                more = false;
+            }
+            bool rest = false;
+            if (!live && mine < n) {
+                ray = mine;
+                r = make_trace_ray(load3(org, ray), load3(dir, ray));
+                if (r.mode == 3 && wide_covers(r)) {
+                    dist = ANY ? tmax[ray] : 1e8f;
+                    closest = -1;
+                    sp = 1;
+                    cur = 0;
+                    leaf = 0;
+                    live = true;
+                } else {
+                    rest = true;
+                }
+            }
+            if (__any_sync(full, rest)) trace_rest<ANY>(a, org, dir, tmax, ray, rest, false, hit_id, hit_t, occ);
+        }
+        // nodes, until few lanes have one and some wait with a triangle or
+        // could be refilled
+        bool overflow = false;
+        for (;;) {
+            const unsigned inner = __ballot_sync(full, cur >= 0);
+            if (inner == 0u) break;
+            if (__popc(inner) < kInner &&
+                (__any_sync(full, leaf != 0) || (more && __popc(__ballot_sync(full, cur == kWideDone)) >= kRefill)))
+                break;
+            if (cur >= 0) {
+                if (sp > kWideStack - 4) {
+                    overflow = true;
+                    cur = kWideDone;
+                    leaf = 0;
+                } else {
+                    wide_node<false>(a.wide, r, none, dist, stack, sp, cur);
+                    if (cur < 0 && cur != kWideDone && leaf == 0) {
+                        leaf = cur;
+                        cur = stack[--sp];
+                    }
+                }
+            }
+        }
+        // the waiting triangles
+        if (leaf != 0) {
+            float t;
+            int prim;
+            if (wide_leaf<false>(a, r, leaf, dist, t, prim)) {
+                closest = prim;
+                dist = t;
+                if (ANY) cur = kWideDone;
+            }
+            leaf = 0;
+            if (cur < 0 && cur != kWideDone) {
+                leaf = cur;
+                cur = stack[--sp];
+            }
+        }
+        if (__any_sync(full, overflow)) {
+            trace_rest<ANY>(a, org, dir, tmax, ray, overflow, true, hit_id, hit_t, occ);
+            if (overflow) live = false;
+        }
+        if (live && cur == kWideDone && leaf == 0) {
+            if (ANY) {
+                occ[ray] = (uint8_t)(closest >= 0);
+            } else {
+                hit_id[ray] = closest;
+                hit_t[ray] = dist;
+            }
+            live = false;
+        }
+    }
 }
 
 // Prefetching schedule: one thread per ray with the node loads of
@@ -247,6 +414,33 @@ int persistent_grid(const void* kernel) {
     return sms * per_sm;
 }
 
+// One wave of resident warps.  Rays too few for eight warps of 32 per SM are
+// spread thinner over eight warps per SM, so that they do not wait for each
+// other's branches (997 rays on 2048 triangles 76 -> 55 us, 5000 on 1M 237 ->
+// 198 us with the whole launch).  Spreading over all resident warps is slower
+// from 60,000 rays on (88 -> 101 us): full warps share their loads.
+struct WideGrid {
+    unsigned blocks;
+    int group;
+};
+WideGrid wide_grid(int64_t n) {
+    static std::atomic<int> sms[64];  // per device
+    int dev = 0, k = 0;
+    cudaGetDevice(&dev);
+    const bool cached = dev >= 0 && dev < 64;
+    if (cached) k = sms[dev].load(std::memory_order_relaxed);
+    if (k == 0) {
+        cudaDeviceGetAttribute(&k, cudaDevAttrMultiProcessorCount, dev);
+        if (k <= 0) k = 1;
+        if (cached) sms[dev].store(k, std::memory_order_relaxed);
+    }
+    const int64_t warps = (int64_t)k * kWideBlocksPerSM * (kWideBlock / 32);
+    const int64_t thin = (int64_t)k * 8;
+    const int64_t group = std::min<int64_t>(32, (n + thin - 1) / thin);
+    const int64_t used = std::min(warps, (n + group - 1) / group);
+    return WideGrid{(unsigned)((used + kWideBlock / 32 - 1) / (kWideBlock / 32)), (int)group};
+}
+
 }  // namespace
 
 cudaError_t launch_pack_nodes(const float* bounds, const int32_t* hit, int64_t M, float4* nodes,
@@ -265,6 +459,11 @@ cudaError_t launch_trace_closest(DeviceAccel a, const float* org, const float* d
     const unsigned g = grid_for(n, kTraceBlock);
     if (a.M > 0 && schedule == ZGL_TRACE_PREFETCH) {
         trace_prefetch_kernel<false><<<g, kTraceBlock, 0, s>>>(a, org, dir, nullptr, n, hit_id, hit_t, nullptr);
+        return cudaGetLastError();
+    }
+    if (a.wide && schedule == ZGL_TRACE_AUTO) {
+        const WideGrid g = wide_grid(n);
+        trace_wide_kernel<false><<<g.blocks, kWideBlock, 0, s>>>(a, org, dir, nullptr, n, g.group, hit_id, hit_t, nullptr);
         return cudaGetLastError();
     }
     if (a.M == 0 || schedule != ZGL_TRACE_PERSISTENT || counter == nullptr) {
@@ -288,6 +487,11 @@ cudaError_t launch_trace_any(DeviceAccel a, const float* org, const float* dir, 
     const unsigned g = grid_for(n, kTraceBlock);
     if (a.M > 0 && schedule == ZGL_TRACE_PREFETCH) {
         trace_prefetch_kernel<true><<<g, kTraceBlock, 0, s>>>(a, org, dir, tmax, n, nullptr, nullptr, occ);
+        return cudaGetLastError();
+    }
+    if (a.wide && schedule == ZGL_TRACE_AUTO) {
+        const WideGrid g = wide_grid(n);
+        trace_wide_kernel<true><<<g.blocks, kWideBlock, 0, s>>>(a, org, dir, tmax, n, g.group, nullptr, nullptr, occ);
         return cudaGetLastError();
     }
     if (a.M == 0 || schedule != ZGL_TRACE_PERSISTENT || counter == nullptr) {
@@ -445,6 +649,18 @@ int host_threads() {
     return n == 0 ? 1 : (int)n;
 }
 
+// Device memory of a scope.
+template <class T>
+struct DevicePtr {
+    T* p = nullptr;
+    explicit DevicePtr(size_t n) { ZGL_CUDA(cudaMalloc(&p, sizeof(T) * std::max<size_t>(n, 1))); }
+    ~DevicePtr() {
+        if (p) cudaFree(p);
+    }
+    DevicePtr(const DevicePtr&) = delete;
+    DevicePtr& operator=(const DevicePtr&) = delete;
+};
+
 // Builds the MTBVH on the host and uploads node records and triangles to the
 // current device.  Throws zgl::Error.
 zgl_accel* accel_create(const float* vertices, const uint32_t* indices, int64_t ntri) {
@@ -479,6 +695,19 @@ zgl_accel* accel_create(const float* vertices, const uint32_t* indices, int64_t 
                 tris[3 * t + 2] = make_float4(acz, 0.0f, 0.0f, 0.0f);
             }
             ZGL_CUDA(cudaMemcpy(a->d_tris, tris.data(), sizeof(float4) * tris.size(), cudaMemcpyHostToDevice));
+            if (a->ntri > 1) {
+                std::vector<float4> dfs((size_t)a->M * 2);
+                std::vector<float> l2((size_t)a->M);
+                host_dfs(a->host, dfs.data(), l2.data());
+                DevicePtr<float> d_l2(l2.size());
+                ZGL_CUDA(cudaMalloc(&a->d_dfs, sizeof(float4) * dfs.size()));
+                ZGL_CUDA(cudaMemcpy(a->d_dfs, dfs.data(), sizeof(float4) * dfs.size(), cudaMemcpyHostToDevice));
+                ZGL_CUDA(cudaMemcpy(d_l2.p, l2.data(), sizeof(float) * l2.size(), cudaMemcpyHostToDevice));
+                ZGL_CUDA(cudaMalloc(&a->d_wide, sizeof(float4) * 4 * (a->ntri - 1)));
+                ZGL_CUDA(cudaMalloc(&a->d_wtris, sizeof(float4) * 4 * a->ntri));
+                build_wide(a, d_l2.p, nullptr, 0);
+                ZGL_CUDA(cudaDeviceSynchronize());
+            }
             ZGL_CUDA(cudaDeviceSynchronize());
             ZGL_CUDA(cudaFree(d_bounds));
             ZGL_CUDA(cudaFree(d_hit));
@@ -497,7 +726,6 @@ zgl_accel* accel_create_device(const float* vertices, int64_t nv, const uint32_t
     uint32_t* d_i = nullptr;
     try {
         ZGL_CUDA(cudaGetDevice(&a->device));
-        ZGL_CUDA(cudaMalloc(&a->d_counter, 256));
         a->ntri = ntri;
         a->M = ntri > 0 ? 2 * ntri - 1 : 0;
         a->device_built = true;
@@ -515,11 +743,26 @@ zgl_accel* accel_create_device(const float* vertices, int64_t nv, const uint32_t
                 ZGL_CUDA(cudaMemcpyAsync(d_i, indices, sizeof(uint32_t) * 3 * ntri, cudaMemcpyHostToDevice, s));
                 idx = d_i;
             }
-            ZGL_CUDA(cudaMalloc(&a->d_nodes, sizeof(float4) * 12 * a->M));
-            ZGL_CUDA(cudaMalloc(&a->d_tris, sizeof(float4) * 3 * a->ntri));
-            ZGL_CUDA(cudaMalloc(&a->d_bounds, sizeof(float) * 6 * a->M));
-            ZGL_CUDA(cudaMalloc(&a->d_hit, sizeof(int32_t) * 18 * a->M));
-            build_bvh_device(v, nv, idx, ntri, small, a->d_nodes, a->d_tris, a->d_bounds, a->d_hit, s);
+            Arena arena;
+            for (int pass = 0; pass < 2; pass++) {
+                arena.bytes = 0;
+                arena.take(a->d_counter, 32);
+                arena.take(a->d_nodes, 12 * a->M);
+                arena.take(a->d_tris, 3 * ntri);
+                arena.take(a->d_dfs, 2 * a->M);
+                arena.take(a->d_hit, 18 * a->M);
+                if (ntri > 1) {
+                    arena.take(a->d_wide, 4 * (ntri - 1));
+                    arena.take(a->d_wtris, 4 * ntri);
+                }
+                if (pass == 0) {
+                    ZGL_CUDA(cudaMalloc(&a->d_arena, arena.bytes));
+                    arena.base = static_cast<char*>(a->d_arena);
+                }
+            }
+            build_bvh_device(v, nv, idx, small, a, s);
+        } else {
+            ZGL_CUDA(cudaMalloc(&a->d_counter, 256));
         }
     } catch (...) {
         cudaStreamSynchronize(s);
@@ -535,11 +778,17 @@ zgl_accel* accel_create_device(const float* vertices, int64_t nv, const uint32_t
 
 void accel_free(zgl_accel* a) {
     if (!a) return;
-    if (a->d_bounds) cudaFree(a->d_bounds);
-    if (a->d_hit) cudaFree(a->d_hit);
-    if (a->d_counter) cudaFree(a->d_counter);
-    if (a->d_nodes) cudaFree(a->d_nodes);
-    if (a->d_tris) cudaFree(a->d_tris);
+    if (a->d_arena) {
+        cudaFree(a->d_arena);
+    } else {
+        if (a->d_dfs) cudaFree(a->d_dfs);
+        if (a->d_hit) cudaFree(a->d_hit);
+        if (a->d_wide) cudaFree(a->d_wide);
+        if (a->d_wtris) cudaFree(a->d_wtris);
+        if (a->d_counter) cudaFree(a->d_counter);
+        if (a->d_nodes) cudaFree(a->d_nodes);
+        if (a->d_tris) cudaFree(a->d_tris);
+    }
     if (a->d_stage) cudaFree(a->d_stage);
     delete a;
 }
@@ -626,7 +875,7 @@ zgl_status zgl_accel_export(const zgl_accel* accel, float* bounds, int32_t* hit_
     if (accel->M > 0 && (!bounds || !hit_table))
         fail(ZGL_ERR_INVALID_ARG, "zgl_accel_export: NULL output array");
     if (accel->M > 0 && accel->device_built) {
-        ZGL_CUDA(cudaMemcpy(bounds, accel->d_bounds, sizeof(float) * accel->M * 6, cudaMemcpyDeviceToHost));
+        export_bounds(accel->d_dfs, accel->M, bounds);
         ZGL_CUDA(cudaMemcpy(hit_table, accel->d_hit, sizeof(int32_t) * accel->M * 18, cudaMemcpyDeviceToHost));
     } else if (accel->M > 0) {
         std::memcpy(bounds, accel->host.bounds.data(), sizeof(float) * accel->M * 6);

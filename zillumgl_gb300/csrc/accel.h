@@ -14,6 +14,38 @@
 //                                   (ab = b - a and ac = c - a evaluated on the
 //                                   host in float32, exactly the values the
 //                                   ray-triangle test forms, intersection.glsl:68-69)
+//   dfs nodes     float4[M][2]      one record per node in DFS pre-order:
+//                                     [0] = pMin.xyz, subtree size, or
+//                                           prim | 0x80000000 at a leaf
+//                                     [1] = pMax.xyz, leaves before the node
+//                                           | 0x80000000 at odd depths
+//   wide tree     uint32[ntri-1][16] two binary levels per 64-byte node: the
+//                                   binary inner node of even depth with
+//                                   DFS index k is wide node k - (leaves
+//                                   before k), so no index has to be
+//                                   allocated (odd-depth slots stay unused).
+//                                   Children: both of the first binary child
+//                                   (slots 0, 1), both of the second (2, 3);
+//                                   a binary child that is a leaf sits in the
+//                                   first slot of its pair.
+//                                     [0..2] grid origin - 2^23 step, xyz
+//                                            (floats)
+//                                     [3]    float exponents of the grid
+//                                            steps (x low byte, y, z) and of
+//                                            the largest squared triangle box
+//                                            diagonal below, rounded up
+//                                     [4..7] child references: wide node,
+//                                            ~leaf slot, or 0 (empty)
+//                                     [8..13] lo.x hi.x lo.y hi.y lo.z hi.z
+//                                            of the children in grid steps
+//                                            from the origin, a byte each,
+//                                            rounded outwards
+//                                     [14]   3 bits per face: bit 0 / 1 the
+//                                            first / second pair in reverse
+//                                            order, bit 2 the second pair
+//                                            first
+//   wide tris     float4[ntri][4]   in DFS leaf order: a.xyz ab.x | ab.yz
+//                                   ac.xy | ac.z prim box lo.xy | lo.z hi.xyz
 #pragma once
 
 #include <cuda_runtime.h>
@@ -27,14 +59,19 @@ struct zgl_accel {
     int64_t ntri = 0;
     int64_t M = 0;
     zgl::HostBVH host;
+    // device-built trees: the one allocation behind the arrays below
+    void* d_arena = nullptr;
     float4* d_nodes = nullptr;  // 6*M*2
     float4* d_tris = nullptr;   // ntri*3
-    // set when the tree was built on the device: the PackedBVH arrays stay
-    // in device memory (bounds float[M*6], hit table int32[6*M*3]) and
-    // `host` is empty
+    // set when the tree was built on the device: the PackedBVH stays in
+    // device memory (bounds in d_dfs, hit table int32[6*M*3]) and `host` is
+    // empty
     bool device_built = false;
-    float* d_bounds = nullptr;
+    float4* d_dfs = nullptr;  // M*2
     int32_t* d_hit = nullptr;
+    // wide tree (ntri >= 2)
+    float4* d_wide = nullptr;   // (ntri-1)*4
+    float4* d_wtris = nullptr;  // ntri*4
     // work counter of the persistent trace kernels (reset before each launch;
     // launches of one handle are serialised on its caller's stream)
     unsigned long long* d_counter = nullptr;
@@ -46,14 +83,31 @@ struct zgl_accel {
 
 namespace zgl {
 
+// Lays arrays out in one allocation: a first pass with base = null measures,
+// a second one hands out the addresses.  A cudaMalloc costs 30-35 us and a
+// cudaFree 15-35 us whatever the size is, on top of 0.7 ms per GB freed.
+struct Arena {
+    char* base = nullptr;
+    size_t bytes = 0;
+    template <class T>
+    void take(T*& p, size_t n) {
+        p = base ? reinterpret_cast<T*>(base + bytes) : nullptr;
+        bytes += (n * sizeof(T) + 255) & ~size_t(255);
+    }
+};
+
 struct DeviceAccel {
     const float4* nodes;
     const float4* tris;
     int32_t M;
+    // wide tree; null where there is none (fewer than two triangles)
+    const float4* wide = nullptr;
+    const float4* wtris = nullptr;
+    const float4* dfs = nullptr;
 };
 
 inline DeviceAccel device_view(const zgl_accel* a) {
-    return DeviceAccel{a->d_nodes, a->d_tris, (int32_t)a->M};
+    return DeviceAccel{a->d_nodes, a->d_tris, (int32_t)a->M, a->d_wide, a->d_wtris, a->d_dfs};
 }
 
 // Kernel launchers (accel.cu).  All pointers are device pointers.
@@ -77,8 +131,16 @@ zgl_accel* accel_create(const float* vertices, const uint32_t* indices, int64_t 
 // pageable host arrays.  `small` = 0 selects the default subtree threshold.
 zgl_accel* accel_create_device(const float* vertices, int64_t nv, const uint32_t* indices, int64_t ntri,
                                int small, cudaStream_t s);
-void build_bvh_device(const float* v, int64_t nv, const uint32_t* idx, int64_t ntri, int small, float4* nodes,
-                      float4* tris, float* bounds, int32_t* hit, cudaStream_t s);
+// Fills d_nodes, d_tris, d_dfs, d_hit and the wide tree.  Synchronous on `s`.
+void build_bvh_device(const float* v, int64_t nv, const uint32_t* idx, int small, zgl_accel* a, cudaStream_t s);
+// Wide tree of an accelerator from its dfs nodes (wide_build.cu) into d_wide
+// and d_wtris, unless the device word `err` (may be null) is set.
+// Asynchronous on `s`.
+void build_wide(zgl_accel* a, const float* l2, const uint32_t* err, cudaStream_t s);
+// dfs nodes and l2 of a host-built tree, as float4[M*2] and float[M].
+void host_dfs(const HostBVH& h, float4* dfs, float* l2);
+// PackedBVH bounds float[M*6] of dfs nodes into host memory.
+void export_bounds(const float4* dfs, int64_t M, float* out);
 int gpu_build_default_small();
 int gpu_build_max_small();
 // Device address of p (itself for device/managed memory, the mapped address

@@ -75,6 +75,7 @@ struct SegAcc {
     uint32_t hi[kBuckets][3];
     unsigned long long zlo[3], zhi[3];
     uint32_t child[2][12];  // per child: centroid lo3 hi3, box lo3 hi3 (ordered keys)
+    uint32_t l2;            // bits of the largest squared box diagonal (>= 0)
     int32_t splitb, nleft;
 };
 
@@ -86,7 +87,8 @@ struct Counters {
 
 struct Out {
     float4* nodes;     // [6][M][2]
-    float* bounds;     // [M][6]
+    float4* dfs;       // [M][2]
+    float* l2;         // [M]
     int32_t* hit;      // [6][M][3]
     int64_t M;
 };
@@ -146,10 +148,19 @@ __device__ __forceinline__ float box_area(const float lo[3], const float hi[3]) 
     return 2.0f * (x * y + y * z + z * x);
 }
 
+// Squared diagonal of a box (never NaN: coordinates lie within +-1e8).
+__device__ __forceinline__ float diag2(const float lo[3], const float hi[3]) {
+    float x = hi[0] - lo[0], y = hi[1] - lo[1], z = hi[2] - lo[2];
+    return x * x + y * y + z * z;
+}
+
 // Writes node `offset` (bounds lo/hi, prim or -1, subtree size) into face
 // f's table at index pos; lanes f = 0..5 of the caller each write one face.
+// Face 0's lane also writes the DFS record: `leaves` leaves come before the
+// node, `odd` is its depth's parity.
 __device__ __forceinline__ void write_entry(const Out& o, int f, int32_t pos, int32_t offset, int32_t prim,
-                                            int32_t size, const float lo[3], const float hi[3]) {
+                                            int32_t size, int32_t leaves, int odd, const float lo[3],
+                                            const float hi[3]) {
     int64_t e = (int64_t)f * o.M + pos;
     o.nodes[2 * e + 0] = make_float4(lo[0], lo[1], lo[2], __int_as_float(prim));
     o.nodes[2 * e + 1] = make_float4(hi[0], hi[1], hi[2], __int_as_float(pos + size));
@@ -157,9 +168,10 @@ __device__ __forceinline__ void write_entry(const Out& o, int f, int32_t pos, in
     o.hit[3 * e + 1] = prim;
     o.hit[3 * e + 2] = pos + size;
     if (f == 0) {
-        float* b = o.bounds + 6 * (int64_t)offset;
-        b[0] = lo[0]; b[1] = lo[1]; b[2] = lo[2];
-        b[3] = hi[0]; b[4] = hi[1]; b[5] = hi[2];
+        const uint32_t w0 = prim < 0 ? (uint32_t)size : ((uint32_t)prim | 0x80000000u);
+        const uint32_t w1 = (uint32_t)leaves | ((uint32_t)odd << 31);
+        o.dfs[2 * (int64_t)offset + 0] = make_float4(lo[0], lo[1], lo[2], __uint_as_float(w0));
+        o.dfs[2 * (int64_t)offset + 1] = make_float4(hi[0], hi[1], hi[2], __uint_as_float(w1));
     }
 }
 
@@ -392,6 +404,7 @@ __global__ void acc_init_kernel(SegAcc* acc, int32_t nseg) {
         A.zlo[threadIdx.x] = ~0ull;
         A.zhi[threadIdx.x] = ~0ull;
     }
+    if (threadIdx.x == 0) A.l2 = 0u;
     if (threadIdx.x < 2) {
         uint32_t* c = A.child[threadIdx.x];
         for (int k = 0; k < 3; k++) {
@@ -409,6 +422,7 @@ __global__ void __launch_bounds__(kLevelBlock) level_bin_kernel(const Seg* __res
                                                                SegAcc* acc, uint32_t* __restrict__ tileHist) {
     __shared__ uint32_t scnt[kBuckets], slo[kBuckets][3], shi[kBuckets][3];
     __shared__ unsigned long long szlo[3], szhi[3];
+    __shared__ uint32_t sl2;
     const Tile tile = tiles[blockIdx.x];
     const Seg S = segs[tile.seg];
     if (threadIdx.x < kBuckets) {
@@ -422,6 +436,8 @@ __global__ void __launch_bounds__(kLevelBlock) level_bin_kernel(const Seg* __res
         szlo[threadIdx.x] = ~0ull;
         szhi[threadIdx.x] = ~0ull;
     }
+    if (threadIdx.x == 0) sl2 = 0u;
+    float l2 = 0.0f;
     __syncthreads();
     const float mn = S.ext[S.dim], mx = S.ext[3 + S.dim];
     const int32_t end = min(S.r, tile.start + kTile - 1);
@@ -431,6 +447,7 @@ __global__ void __launch_bounds__(kLevelBlock) level_bin_kernel(const Seg* __res
         rec_box(p, lo, hi);
         int b = bucket_of(rec_centroid(p, S.dim), mn, mx);
         atomicAdd(&scnt[b], 1u);
+        l2 = fmaxf(l2, diag2(lo, hi));
         unsigned long long rel = (unsigned long long)(i - S.l);
 #pragma unroll
         for (int k = 0; k < 3; k++) {
@@ -442,8 +459,11 @@ __global__ void __launch_bounds__(kLevelBlock) level_bin_kernel(const Seg* __res
                 atomicMin(&szhi[k], ((unsigned long long)b << 40) | (rel << 1) | (__float_as_uint(hi[k]) >> 31));
         }
     }
+    const uint32_t wl2 = __reduce_max_sync(0xffffffffu, __float_as_uint(l2));
+    if ((threadIdx.x & 31) == 0) atomicMax(&sl2, wl2);
     __syncthreads();
     SegAcc& A = acc[tile.seg];
+    if (threadIdx.x == kLevelBlock - 1) atomicMax(&A.l2, sl2);
     if (threadIdx.x < kBuckets) {
         uint32_t c = scnt[threadIdx.x];
         tileHist[(int64_t)blockIdx.x * kBuckets + threadIdx.x] = c;
@@ -494,8 +514,10 @@ __global__ void __launch_bounds__(kLevelBlock) level_split_kernel(const Seg* __r
             lo[k] = resolve_zero(tl[k], A.zlo[k]);
             hi[k] = resolve_zero(th[k], A.zhi[k]);
         }
-        if (threadIdx.x < 6) write_entry(o, threadIdx.x, S.pos[threadIdx.x], S.offset, -1, 2 * n - 1, lo, hi);
+        if (threadIdx.x < 6)
+            write_entry(o, threadIdx.x, S.pos[threadIdx.x], S.offset, -1, 2 * n - 1, S.l, S.buf, lo, hi);
         if (threadIdx.x == 0) {
+            o.l2[S.offset] = __uint_as_float(A.l2);
             sSplit = split;
             sNleft = nl;
             A.splitb = split;
@@ -702,7 +724,7 @@ __device__ void emit_tiny(const Seg& S, PrimRec* const bufs[2], const Out& o) {
             PrimRec p = in[S.l];
             float lo[3], hi[3];
             rec_box(p, lo, hi);
-            write_entry(o, lane, S.pos[lane], S.offset, rec_id(p), 1, lo, hi);
+            write_entry(o, lane, S.pos[lane], S.offset, rec_id(p), 1, S.l, S.buf, lo, hi);
         }
         return;
     }
@@ -721,15 +743,16 @@ __device__ void emit_tiny(const Seg& S, PrimRec* const bufs[2], const Out& o) {
         rec_box(B, blo, bhi);
     }
     const int f = lane;
-    write_entry(o, f, S.pos[f], S.offset, -1, 3, lo, hi);
+    write_entry(o, f, S.pos[f], S.offset, -1, 3, S.l, S.buf, lo, hi);
+    if (f == 0) o.l2[S.offset] = fmaxf(diag2(alo, ahi), diag2(blo, bhi));
     int axis = f >> 1;
     bool greater = (f & 1) == 0;
     float cl = (alo[axis] + ahi[axis]) * 0.5f, cr = (blo[axis] + bhi[axis]) * 0.5f;
     bool aFirst = greater ? (cl > cr) : (cl < cr);
     int32_t pa = S.pos[f] + (aFirst ? 1 : 2), pb = S.pos[f] + (aFirst ? 2 : 1);
     // the two leaves' bounds are written by face 0's lane, like every node's
-    write_entry(o, f, pa, S.offset + 1, rec_id(A), 1, alo, ahi);
-    write_entry(o, f, pb, S.offset + 2, rec_id(B), 1, blo, bhi);
+    write_entry(o, f, pa, S.offset + 1, rec_id(A), 1, S.l, 1 - S.buf, alo, ahi);
+    write_entry(o, f, pb, S.offset + 2, rec_id(B), 1, S.l + 1, 1 - S.buf, blo, bhi);
 }
 
 __global__ void __launch_bounds__(kSubtreeBlock) subtree_kernel(const Seg* __restrict__ list, PrimRec* buf0,
@@ -772,12 +795,14 @@ __global__ void __launch_bounds__(kSubtreeBlock) subtree_kernel(const Seg* __res
                 ws.zhi[lane - kBuckets] = 0xffffffffu;
             }
             __syncwarp();
+            float l2 = 0.0f;
             for (int32_t i = S.l + lane; i <= S.r; i += 32) {
                 PrimRec p = in[i];
                 float lo[3], hi[3];
                 rec_box(p, lo, hi);
                 int b = bucket_of(rec_centroid(p, S.dim), mn, mx);
                 atomicAdd(&ws.cnt[b], 1u);
+                l2 = fmaxf(l2, diag2(lo, hi));
                 uint32_t rel = (uint32_t)(i - S.l);
 #pragma unroll
                 for (int k = 0; k < 3; k++) {
@@ -787,7 +812,7 @@ __global__ void __launch_bounds__(kSubtreeBlock) subtree_kernel(const Seg* __res
                     if (hi[k] == 0.0f) atomicMin(&ws.zhi[k], ((uint32_t)b << 13) | (rel << 1) | (__float_as_uint(hi[k]) >> 31));
                 }
             }
-            __syncwarp();
+            const uint32_t wl2 = __reduce_max_sync(full, __float_as_uint(l2));
             uint32_t lk[3], hk[3], tl[3], th[3], nleftU;
             const int bb = lane & 15;
             for (int k = 0; k < 3; k++) {
@@ -808,7 +833,8 @@ __global__ void __launch_bounds__(kSubtreeBlock) subtree_kernel(const Seg* __res
                     lo[k] = resolve_zero(tl[k], zl == 0xffffffffu ? ~0ull : (unsigned long long)zl);
                     hi[k] = resolve_zero(th[k], zh == 0xffffffffu ? ~0ull : (unsigned long long)zh);
                 }
-                write_entry(o, lane, S.pos[lane], S.offset, -1, 2 * n - 1, lo, hi);
+                write_entry(o, lane, S.pos[lane], S.offset, -1, 2 * n - 1, S.l, S.buf, lo, hi);
+                if (lane == 0) o.l2[S.offset] = __uint_as_float(wl2);
             }
             // stable partition: left buckets in order, right buckets reversed
             uint32_t ck[2][12];
@@ -873,13 +899,49 @@ __global__ void __launch_bounds__(kSubtreeBlock) subtree_kernel(const Seg* __res
     }
 }
 
-template <class T>
-struct DevBuf {
-    T* p = nullptr;
-    ~DevBuf() {
-        if (p) cudaFree(p);
+// The build's working memory, one allocation.
+struct Scratch {
+    void* p = nullptr;
+    PrimRec *rec0, *rec1;
+    Counters* ctr;
+    uint32_t* rootExt;
+    float* l2;
+    Seg *big[2], *smallList;
+    Tile* tiles[2];
+    int32_t* tile0[2];
+    SegAcc* acc;
+    uint32_t* tileHist;
+    int2* tileOff;
+
+    Scratch(int64_t ntri, int small) {
+        const int64_t maxBig = ntri / small + 2;
+        const int64_t maxTiles = (ntri + kTile - 1) / kTile + maxBig;
+        Arena a;
+        for (int pass = 0; pass < 2; pass++) {
+            a.bytes = 0;
+            a.take(rec0, ntri);
+            a.take(rec1, ntri);
+            a.take(ctr, 1);
+            a.take(rootExt, 6);
+            a.take(l2, 2 * ntri);
+            for (int i = 0; i < 2; i++) {
+                a.take(big[i], maxBig);
+                a.take(tiles[i], maxTiles);
+                a.take(tile0[i], maxBig);
+            }
+            a.take(smallList, ntri + 1);
+            a.take(acc, maxBig);
+            a.take(tileHist, maxTiles * kBuckets);
+            a.take(tileOff, maxTiles);
+            if (pass == 0) {
+                ZGL_CUDA(cudaMalloc(&p, a.bytes));
+                a.base = static_cast<char*>(p);
+            }
+        }
     }
-    void alloc(size_t n) { ZGL_CUDA(cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(T))); }
+    ~Scratch() { cudaFree(p); }
+    Scratch(const Scratch&) = delete;
+    Scratch& operator=(const Scratch&) = delete;
 };
 
 }  // namespace
@@ -887,48 +949,23 @@ struct DevBuf {
 int gpu_build_default_small() { return kDefaultSmall; }
 int gpu_build_max_small() { return kMaxSmall; }
 
-// Builds the MTBVH of `ntri` triangles on the current device (vertices and
-// indices are device-accessible).  Fills nodes (float4[6][M][2]), tris
-// (float4[ntri][3]), bounds (float[M][6]) and hit (int32[6][M][3]).
-// Synchronous on `s`; throws zgl::Error.
-void build_bvh_device(const float* v, int64_t nv, const uint32_t* idx, int64_t ntri, int small,
-                      float4* nodes, float4* tris, float* bounds, int32_t* hit, cudaStream_t s) {
+// Builds the MTBVH of the accelerator's triangles on the current device
+// (vertices and indices are device-accessible): d_nodes, d_tris, d_dfs, d_hit
+// and the wide tree.  Synchronous on `s`; throws zgl::Error.
+void build_bvh_device(const float* v, int64_t nv, const uint32_t* idx, int small, zgl_accel* a, cudaStream_t s) {
+    const int64_t ntri = a->ntri;
     if (ntri <= 0) return;
     if (small <= 0) small = kDefaultSmall;
     small = std::max(8, std::min(small, kMaxSmall));
-    const int64_t M = 2 * ntri - 1;
-    Out o{nodes, bounds, hit, M};
-
-    DevBuf<PrimRec> rec0, rec1;
-    DevBuf<Counters> ctr;
-    DevBuf<uint32_t> rootExt;
-    rec0.alloc(ntri);
-    rec1.alloc(ntri);
-    ctr.alloc(1);
-    rootExt.alloc(6);
-    const int64_t maxBig = ntri / small + 2;
-    const int64_t maxTiles = (ntri + kTile - 1) / kTile + maxBig;
-    DevBuf<Seg> big[2], smallList;
-    DevBuf<Tile> tiles[2];
-    DevBuf<int32_t> tile0[2];
-    DevBuf<SegAcc> acc;
-    DevBuf<uint32_t> tileHist;
-    DevBuf<int2> tileOff;
-    for (int i = 0; i < 2; i++) {
-        big[i].alloc(maxBig);
-        tiles[i].alloc(maxTiles);
-        tile0[i].alloc(maxBig);
-    }
-    smallList.alloc(ntri + 1);
-    acc.alloc(maxBig);
-    tileHist.alloc(maxTiles * kBuckets);
-    tileOff.alloc(maxTiles);
+    Scratch w(ntri, small);
+    Out o{a->d_nodes, a->d_dfs, w.l2, a->d_hit, a->M};
+    float4* const tris = a->d_tris;
 
     int dev = 0, sms = 1;
     ZGL_CUDA(cudaGetDevice(&dev));
     ZGL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
 
-    ZGL_CUDA(cudaMemsetAsync(ctr.p, 0, sizeof(Counters), s));
+    ZGL_CUDA(cudaMemsetAsync(w.ctr, 0, sizeof(Counters), s));
     {
         uint32_t init[6];
         float lo = 1e8f, hi = -1e8f;
@@ -941,42 +978,42 @@ void build_bvh_device(const float* v, int64_t nv, const uint32_t* idx, int64_t n
             init[k] = hkey(ul);
             init[3 + k] = hkey(uh);
         }
-        ZGL_CUDA(cudaMemcpyAsync(rootExt.p, init, sizeof(init), cudaMemcpyHostToDevice, s));
+        ZGL_CUDA(cudaMemcpyAsync(w.rootExt, init, sizeof(init), cudaMemcpyHostToDevice, s));
     }
     int64_t work = std::max<int64_t>(ntri, 3 * nv);
     int grid = (int)std::min<int64_t>((work + 255) / 256, (int64_t)sms * 16);
-    setup_kernel<<<grid, 256, 0, s>>>(v, nv, idx, ntri, rec0.p, tris, rootExt.p, ctr.p);
+    setup_kernel<<<grid, 256, 0, s>>>(v, nv, idx, ntri, w.rec0, tris, w.rootExt, w.ctr);
     ZGL_CUDA(cudaGetLastError());
     Counters h{};
-    ZGL_CUDA(cudaMemcpyAsync(&h, ctr.p, sizeof(Counters), cudaMemcpyDeviceToHost, s));
+    ZGL_CUDA(cudaMemcpyAsync(&h, w.ctr, sizeof(Counters), cudaMemcpyDeviceToHost, s));
     ZGL_CUDA(cudaStreamSynchronize(s));
     if (h.err & kErrIndex) fail(ZGL_ERR_INVALID_ARG, "bvh build: triangle index out of range");
     if (h.err & kErrVertex)
         fail(ZGL_ERR_INVALID_ARG, "bvh build: vertex component NaN, infinite or beyond +-1e8");
 
-    root_kernel<<<1, 256, 0, s>>>(rootExt.p, (int32_t)ntri, small, big[0].p, tiles[0].p, smallList.p, ctr.p);
+    root_kernel<<<1, 256, 0, s>>>(w.rootExt, (int32_t)ntri, small, w.big[0], w.tiles[0], w.smallList, w.ctr);
     ZGL_CUDA(cudaGetLastError());
-    ZGL_CUDA(cudaMemsetAsync(tile0[0].p, 0, sizeof(int32_t), s));
-    ZGL_CUDA(cudaMemcpyAsync(&h, ctr.p, sizeof(Counters), cudaMemcpyDeviceToHost, s));
+    ZGL_CUDA(cudaMemsetAsync(w.tile0[0], 0, sizeof(int32_t), s));
+    ZGL_CUDA(cudaMemcpyAsync(&h, w.ctr, sizeof(Counters), cudaMemcpyDeviceToHost, s));
     ZGL_CUDA(cudaStreamSynchronize(s));
 
-    PrimRec* bufs[2] = {rec0.p, rec1.p};
+    PrimRec* bufs[2] = {w.rec0, w.rec1};
     int cur = 0, level = 0;
     while (h.nbig > 0) {
         const int32_t nbig = (int32_t)h.nbig, ntiles = (int32_t)h.ntiles;
         const PrimRec* in = bufs[level & 1];
         PrimRec* outb = bufs[(level + 1) & 1];
-        acc_init_kernel<<<nbig, 32, 0, s>>>(acc.p, nbig);
-        level_bin_kernel<<<ntiles, kLevelBlock, 0, s>>>(big[cur].p, tiles[cur].p, in, acc.p, tileHist.p);
-        level_split_kernel<<<nbig, kLevelBlock, 0, s>>>(big[cur].p, acc.p, tiles[cur].p, tileHist.p, tileOff.p,
-                                                        tile0[cur].p, o, ctr.p);
-        level_scatter_kernel<<<ntiles, kLevelBlock, 0, s>>>(big[cur].p, acc.p, tiles[cur].p, tileOff.p, in, outb);
+        acc_init_kernel<<<nbig, 32, 0, s>>>(w.acc, nbig);
+        level_bin_kernel<<<ntiles, kLevelBlock, 0, s>>>(w.big[cur], w.tiles[cur], in, w.acc, w.tileHist);
+        level_split_kernel<<<nbig, kLevelBlock, 0, s>>>(w.big[cur], w.acc, w.tiles[cur], w.tileHist, w.tileOff,
+                                                        w.tile0[cur], o, w.ctr);
+        level_scatter_kernel<<<ntiles, kLevelBlock, 0, s>>>(w.big[cur], w.acc, w.tiles[cur], w.tileOff, in, outb);
         // next level's counters start at zero (the subtree count accumulates)
-        ZGL_CUDA(cudaMemsetAsync(ctr.p, 0, 2 * sizeof(uint32_t), s));
-        level_finalize_kernel<<<nbig, 32, 0, s>>>(big[cur].p, acc.p, nbig, small, big[1 - cur].p,
-                                                  tiles[1 - cur].p, tile0[1 - cur].p, smallList.p, ctr.p);
+        ZGL_CUDA(cudaMemsetAsync(w.ctr, 0, 2 * sizeof(uint32_t), s));
+        level_finalize_kernel<<<nbig, 32, 0, s>>>(w.big[cur], w.acc, nbig, small, w.big[1 - cur],
+                                                  w.tiles[1 - cur], w.tile0[1 - cur], w.smallList, w.ctr);
         ZGL_CUDA(cudaGetLastError());
-        ZGL_CUDA(cudaMemcpyAsync(&h, ctr.p, sizeof(Counters), cudaMemcpyDeviceToHost, s));
+        ZGL_CUDA(cudaMemcpyAsync(&h, w.ctr, sizeof(Counters), cudaMemcpyDeviceToHost, s));
         ZGL_CUDA(cudaStreamSynchronize(s));
         if (h.err) break;
         cur = 1 - cur;
@@ -986,10 +1023,11 @@ void build_bvh_device(const float* v, int64_t nv, const uint32_t* idx, int64_t n
     if (h.nsmall > 0) {
         int warps = (int)std::min<int64_t>(h.nsmall, (int64_t)sms * 64);
         int blocks = (warps + kSubtreeBlock / 32 - 1) / (kSubtreeBlock / 32);
-        subtree_kernel<<<blocks, kSubtreeBlock, 0, s>>>(smallList.p, rec0.p, rec1.p, o, ctr.p);
+        subtree_kernel<<<blocks, kSubtreeBlock, 0, s>>>(w.smallList, w.rec0, w.rec1, o, w.ctr);
         ZGL_CUDA(cudaGetLastError());
     }
-    ZGL_CUDA(cudaMemcpyAsync(&h, ctr.p, sizeof(Counters), cudaMemcpyDeviceToHost, s));
+    if (ntri > 1) build_wide(a, w.l2, &w.ctr->err, s);
+    ZGL_CUDA(cudaMemcpyAsync(&h, w.ctr, sizeof(Counters), cudaMemcpyDeviceToHost, s));
     ZGL_CUDA(cudaStreamSynchronize(s));
     if (h.err & kErrSplit) fail(ZGL_ERR_STATE, "bvh build: empty split (coordinates beyond the default box)");
     if (h.err & kErrStack) fail(ZGL_ERR_STATE, "bvh build: subtree stack overflow");

@@ -108,12 +108,10 @@ __device__ __forceinline__ bool box_hit(const float4 lo, const float4 hi, const 
     }
 }
 
-// intersectTriangle with precomputed a, ab = b - a, ac = c - a.
-__device__ __forceinline__ bool tri_hit(const float4* __restrict__ tris, int prim,
-                                        const TraceRay& r, float& t) {
-    const float4 t0 = __ldg(tris + 3 * (size_t)prim);
-    const float4 t1 = __ldg(tris + 3 * (size_t)prim + 1);
-    const float4 t2 = __ldg(tris + 3 * (size_t)prim + 2);
+// intersectTriangle with precomputed a, ab = b - a, ac = c - a, in the three
+// float4 of a traversal triangle (a.xyz ab.x | ab.yz ac.xy | ac.z ...).
+__device__ __forceinline__ bool tri_test(const float4 t0, const float4 t1, const float4 t2, const TraceRay& r,
+                                         float& t) {
     const float abx = t0.w, aby = t1.x, abz = t1.y;
     const float acx = t1.z, acy = t1.w, acz = t2.x;
     const float3 d = r.d;
@@ -142,6 +140,11 @@ __device__ __forceinline__ bool tri_hit(const float4* __restrict__ tris, int pri
     return t > 0.0f;
 }
 
+__device__ __forceinline__ bool tri_hit(const float4* __restrict__ tris, int prim,
+                                        const TraceRay& r, float& t) {
+    return tri_test(__ldg(tris + 3 * (size_t)prim), __ldg(tris + 3 * (size_t)prim + 1),
+                    __ldg(tris + 3 * (size_t)prim + 2), r, t);
+}
 // bvhHit (ANY = false): returns the closest primitive or -1 and lowers `dist`.
 // bvhTest (ANY = true): returns 1 at the first t < dist, else 0.
 // The loop index only grows (k = max(miss, k + 1)), so it ends within M steps
