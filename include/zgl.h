@@ -105,17 +105,19 @@ zgl_status zgl_bvh_build_host(const float* vertices, size_t n_vertices,
 /* Trace kernel schedule of an accelerator.  All give identical results;
  * only speed differs.  The reference has one fixed schedule (one invocation
  * per pixel or path, src/integrator/NaivePath.cpp:94-100).
- *   ZGL_TRACE_AUTO (0, default): one thread per ray; a ray with a
- *     direction component below 1e-6 in magnitude (boxHit's near-zero
- *     branch can make it visit tens of thousands of table entries) that has
- *     not finished after 256 entries is finished by its whole warp, 32
- *     consecutive entries at a time.
+ *   ZGL_TRACE_AUTO (0, default): a tree of four children per node in the
+ *     reference's visiting order, resident warps whose lanes take the next
+ *     ray as theirs ends; a ray with a direction component below 1e-6 in
+ *     magnitude (boxHit's near-zero branch can make it visit tens of
+ *     thousands of table entries) that outruns its budget is finished on the
+ *     threaded table by its whole warp, 32 consecutive entries at a time.
  *   ZGL_TRACE_THREAD_PER_RAY (1): one thread per ray, every ray on its own
  *     lane to the end (the reference's schedule).
  *   ZGL_TRACE_PERSISTENT (2): persistent warps that refill idle lanes by
  *     atomic fetch.
- *   ZGL_TRACE_PREFETCH (3): as ZGL_TRACE_AUTO, with every lane requesting
- *     both possible successors of a node ahead. */
+ *   ZGL_TRACE_PREFETCH (3): one thread per ray on the threaded table, every
+ *     lane requesting both possible successors of an entry ahead; long rays
+ *     finished by the warp. */
 enum { ZGL_TRACE_AUTO = 0, ZGL_TRACE_THREAD_PER_RAY = 1, ZGL_TRACE_PERSISTENT = 2, ZGL_TRACE_PREFETCH = 3 };
 zgl_status zgl_accel_set_trace_schedule(zgl_accel* accel, int32_t schedule);
 
@@ -317,7 +319,7 @@ zgl_status zgl_integrator_render_pass(zgl_integrator* integ, void* stream);
 
 /* `passes` consecutive calls of zgl_integrator_render_pass in one go: the
  * frame, sample count and counters end exactly as after those calls.  The
- * path tracer renders all of them in one launch (per-pass radiance in a
+ * path tracer renders all of them together (per-pass radiance in a
  * device scratch buffer of filmW*filmH*3*passes floats kept by the
  * integrator, then added to the frame in pass order), which fills the GPU at
  * small film sizes; the light and triple integrators run one pass at a time.
@@ -383,9 +385,10 @@ typedef struct zgl_render_request {
 } zgl_render_request;
 
 /* Schedule of the batched renderer; 0 picks the default (or, after
- * zgl_batch_autotune, the tuned value).  schedule: ZGL_BATCH_FLAT (one grid of
- * 16x8 pixel tiles over every sample of every request, straight-line path
- * code per thread; the default), ZGL_BATCH_PERSISTENT (persistent warps
+ * zgl_batch_autotune, the tuned value).  schedule: ZGL_BATCH_FLAT (requests
+ * with paths enough run one after the other with ray casts and shading in
+ * separate kernels, the others together in one grid of 16x8 pixel tiles with
+ * straight-line path code per thread; the default), ZGL_BATCH_PERSISTENT (persistent warps
  * with per-bounce path state and path regeneration) or ZGL_BATCH_QUEUE
  * (persistent blocks of 256 threads whose paths put their closest-hit and
  * shadow rays into dense queues in shared memory, traced by the whole block

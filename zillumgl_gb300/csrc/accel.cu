@@ -101,169 +101,37 @@ trace_count_kernel(DeviceAccel a, const float* __restrict__ org, const float* __
     tests[i] = t;
 }
 
-// Rays of a warp that the wide tree's loop leaves out, marked by `want`: the
-// rarer modes one per lane on the wide tree, the others (and those whose
-// stack ran out) on the face table, past kLaneBudget entries with the whole
-// warp.  Every lane calls.
 template <bool ANY>
-static __device__ __noinline__ void trace_rest(DeviceAccel a, const float* org, const float* dir, const float* tmax,
-                                               int64_t i, bool want, bool overflow, int32_t* hit_id, float* hit_t,
-                                               uint8_t* occ) {
-    const TraceRay r = lane_ray(org, dir, i, want);
-    float dist = ANY ? (want ? tmax[i] : 0.0f) : 1e8f;
-    int closest = -1;
-    bool done = !want;
-    if (want && !overflow && wide_covers(r)) {
-        const WideHit h = traverse_wide<ANY, true>(a, r, dist);
-        if (h.ok) {
-            closest = h.id;
-            dist = h.dist;
-            done = true;
+struct RayArrays {
+    static constexpr bool kClosest = !ANY, kAny = ANY;
+    const float *org, *dir, *tmax;
+    int32_t* hit_id;
+    float* hit_t;
+    uint8_t* occ;
+    __device__ __forceinline__ bool any(int) const { return ANY; }
+    __device__ __forceinline__ float3 origin(int i) const { return load3(org, i); }
+    __device__ __forceinline__ float3 direction(int i) const { return load3(dir, i); }
+    __device__ __forceinline__ float limit(int i) const { return ANY ? tmax[i] : 1e8f; }
+    __device__ __forceinline__ void store(int i, int id, float t) const {
+        if (ANY) {
+            occ[i] = (uint8_t)(id >= 0);
+        } else {
+            hit_id[i] = id;
+            hit_t[i] = t;
         }
     }
-    if (!__all_sync(0xffffffffu, done)) {
-        int k = 0;
-        done = done || traverse_lane_m<ANY, false, 0>(a, r, dist, k, closest, kLaneBudget);
-        finish_long_rays<ANY>(a, r, dist, k, closest, done);
+    __device__ __forceinline__ void mark(int i) const {
+        if (ANY) occ[i] = 2;
+        else hit_id[i] = -2;
     }
-    if (!want) return;
-    if (ANY) {
-        occ[i] = (uint8_t)(closest >= 0);
-    } else {
-        hit_id[i] = closest;
-        hit_t[i] = dist;
-    }
-}
+    __device__ __forceinline__ bool marked(int i) const { return ANY ? occ[i] == 2 : hit_id[i] == -2; }
+};
 
-// The default schedule: closest or any hit of every ray on the wide tree.
-//
-// Divergence is what this loop fights.  Rays of one warp visit between a few
-// and 400 nodes (mean 31 on the 4M soup's bounce rays, 4 triangles); one ray
-// per thread to the end kept 5.5 lanes busy and ran at 740 Mrays/s.  So
-//  * the grid is one wave of resident warps, each taking every nwarps-th group
-//    of 32 rays; lanes without a ray are refilled from the sequence once
-//    kRefill of them are idle (no counter in memory, so launches on other
-//    streams and in graphs stay independent).  256 consecutive rays per warp
-//    instead: 1083 Mrays/s, one wave: 1268 (its tails come once a launch);
-//  * a lane that reaches a triangle sets it aside and goes on with the nodes
-//    behind it (a later, larger distance only adds nodes; triangles are still
-//    tested in order).  The warp turns to the waiting triangles when fewer
-//    than kInner lanes have a node left (8 to 24 measured, flat at 16 to 20).
-// 64-byte nodes in two 32-byte loads: with 128-byte nodes of full floats in
-// eight 16-byte loads the L1 was 70% busy (a gather takes a cycle a lane) and
-// the same loop ran at 760 Mrays/s.  48 registers (20 warps of 64 threads per
-// SM) hide more latency than 64 (1192) or 40 (1268 and slower when coherent).
-constexpr int kWideBlock = 64;
-constexpr int kWideBlocksPerSM = 20;
-constexpr int kInner = 16;
-constexpr int kRefill = 8;
-
+// The default schedule: every ray on the wide tree.
 template <bool ANY>
 __global__ void __launch_bounds__(kWideBlock, kWideBlocksPerSM)
-trace_wide_kernel(DeviceAccel a, const float* __restrict__ org, const float* __restrict__ dir,
-                  const float* __restrict__ tmax, int64_t n, int group, int32_t* __restrict__ hit_id,
-                  float* __restrict__ hit_t, uint8_t* __restrict__ occ) {
-    const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const unsigned lt = (1u << lane) - 1u;
-    // ray p of this warp's sequence is ray ((p / 32) * nwarps + warp) * 32 +
-    // p % 32; with fewer rays than that takes, the warp has `group` of them
-    const int64_t warp = blockIdx.x * (int64_t)(kWideBlock / 32) + (threadIdx.x >> 5);
-    const int64_t nwarps = gridDim.x * (int64_t)(kWideBlock / 32);
-    int64_t taken = 0;
-    bool more = warp * group < n;
-    int stack[kWideStack];
-    stack[0] = kWideDone;
-    int64_t ray = 0;
-    TraceRay r;
-    const WidePad none{};
-    float dist = 0.0f;
-    int closest = -1, sp = 1, cur = kWideDone, leaf = 0;
-    bool live = false;
-    for (;;) {
-        // refill the lanes without a ray
-        const unsigned idle = __ballot_sync(full, !live);
-        if (idle == full && !more) break;
-        if (more && __popc(idle) >= kRefill) {
-            const int64_t p = taken + __popc(idle & lt);
-            int64_t mine;
-            if (group == 32) {
-                mine = ((p >> 5) * nwarps + warp) * 32 + (p & 31);
-                taken += __popc(idle);
-                more = ((taken >> 5) * nwarps + warp) * 32 + (taken & 31) < n;
-            } else {
-                mine = p < group ? warp * group + p : n;
-                more = false;
-            }
-            bool rest = false;
-            if (!live && mine < n) {
-                ray = mine;
-                r = make_trace_ray(load3(org, ray), load3(dir, ray));
-                if (r.mode == 3 && wide_covers(r)) {
-                    dist = ANY ? tmax[ray] : 1e8f;
-                    closest = -1;
-                    sp = 1;
-                    cur = 0;
-                    leaf = 0;
-                    live = true;
-                } else {
-                    rest = true;
-                }
-            }
-            if (__any_sync(full, rest)) trace_rest<ANY>(a, org, dir, tmax, ray, rest, false, hit_id, hit_t, occ);
-        }
-        // nodes, until few lanes have one and some wait with a triangle or
-        // could be refilled
-        bool overflow = false;
-        for (;;) {
-            const unsigned inner = __ballot_sync(full, cur >= 0);
-            if (inner == 0u) break;
-            if (__popc(inner) < kInner &&
-                (__any_sync(full, leaf != 0) || (more && __popc(__ballot_sync(full, cur == kWideDone)) >= kRefill)))
-                break;
-            if (cur >= 0) {
-                if (sp > kWideStack - 4) {
-                    overflow = true;
-                    cur = kWideDone;
-                    leaf = 0;
-                } else {
-                    wide_node<false>(a.wide, r, none, dist, stack, sp, cur);
-                    if (cur < 0 && cur != kWideDone && leaf == 0) {
-                        leaf = cur;
-                        cur = stack[--sp];
-                    }
-                }
-            }
-        }
-        // the waiting triangles
-        if (leaf != 0) {
-            float t;
-            int prim;
-            if (wide_leaf<false>(a, r, leaf, dist, t, prim)) {
-                closest = prim;
-                dist = t;
-                if (ANY) cur = kWideDone;
-            }
-            leaf = 0;
-            if (cur < 0 && cur != kWideDone) {
-                leaf = cur;
-                cur = stack[--sp];
-            }
-        }
-        if (__any_sync(full, overflow)) {
-            trace_rest<ANY>(a, org, dir, tmax, ray, overflow, true, hit_id, hit_t, occ);
-            if (overflow) live = false;
-        }
-        if (live && cur == kWideDone && leaf == 0) {
-            if (ANY) {
-                occ[ray] = (uint8_t)(closest >= 0);
-            } else {
-                hit_id[ray] = closest;
-                hit_t[ray] = dist;
-            }
-            live = false;
-        }
-    }
+trace_wide_kernel(const __grid_constant__ DeviceAccel a, const __grid_constant__ RayArrays<ANY> io, int n, int group) {
+    wide_trace(a, io, n, group);
 }
 
 // Prefetching schedule: one thread per ray with the node loads of
@@ -414,17 +282,9 @@ int persistent_grid(const void* kernel) {
     return sms * per_sm;
 }
 
-// One wave of resident warps.  Rays too few for eight warps of 32 per SM are
-// spread thinner over eight warps per SM, so that they do not wait for each
-// other's branches (997 rays on 2048 triangles 76 -> 55 us, 5000 on 1M 237 ->
-// 198 us with the whole launch).  Spreading over all resident warps is slower
-// from 60,000 rays on (88 -> 101 us): full warps share their loads.
-struct WideGrid {
-    unsigned blocks;
-    int group;
-};
-WideGrid wide_grid(int64_t n) {
-    static std::atomic<int> sms[64];  // per device
+// SMs of the current device (cached per device).
+int sm_count() {
+    static std::atomic<int> sms[64];
     int dev = 0, k = 0;
     cudaGetDevice(&dev);
     const bool cached = dev >= 0 && dev < 64;
@@ -434,11 +294,7 @@ WideGrid wide_grid(int64_t n) {
         if (k <= 0) k = 1;
         if (cached) sms[dev].store(k, std::memory_order_relaxed);
     }
-    const int64_t warps = (int64_t)k * kWideBlocksPerSM * (kWideBlock / 32);
-    const int64_t thin = (int64_t)k * 8;
-    const int64_t group = std::min<int64_t>(32, (n + thin - 1) / thin);
-    const int64_t used = std::min(warps, (n + group - 1) / group);
-    return WideGrid{(unsigned)((used + kWideBlock / 32 - 1) / (kWideBlock / 32)), (int)group};
+    return k;
 }
 
 }  // namespace
@@ -462,8 +318,12 @@ cudaError_t launch_trace_closest(DeviceAccel a, const float* org, const float* d
         return cudaGetLastError();
     }
     if (a.wide && schedule == ZGL_TRACE_AUTO) {
-        const WideGrid g = wide_grid(n);
-        trace_wide_kernel<false><<<g.blocks, kWideBlock, 0, s>>>(a, org, dir, nullptr, n, g.group, hit_id, hit_t, nullptr);
+        const int sms = sm_count();
+        for (int64_t at = 0; at < n; at += kWideMaxRays) {
+            const int64_t m = std::min(n - at, kWideMaxRays);
+            const RayArrays<false> io{org + 3 * at, dir + 3 * at, nullptr, hit_id + at, hit_t + at, nullptr};
+            trace_wide_kernel<false><<<wide_blocks(m, sms), kWideBlock, 0, s>>>(a, io, (int)m, wide_group(m, sms));
+        }
         return cudaGetLastError();
     }
     if (a.M == 0 || schedule != ZGL_TRACE_PERSISTENT || counter == nullptr) {
@@ -490,8 +350,12 @@ cudaError_t launch_trace_any(DeviceAccel a, const float* org, const float* dir, 
         return cudaGetLastError();
     }
     if (a.wide && schedule == ZGL_TRACE_AUTO) {
-        const WideGrid g = wide_grid(n);
-        trace_wide_kernel<true><<<g.blocks, kWideBlock, 0, s>>>(a, org, dir, tmax, n, g.group, nullptr, nullptr, occ);
+        const int sms = sm_count();
+        for (int64_t at = 0; at < n; at += kWideMaxRays) {
+            const int64_t m = std::min(n - at, kWideMaxRays);
+            const RayArrays<true> io{org + 3 * at, dir + 3 * at, tmax + at, nullptr, nullptr, occ + at};
+            trace_wide_kernel<true><<<wide_blocks(m, sms), kWideBlock, 0, s>>>(a, io, (int)m, wide_group(m, sms));
+        }
         return cudaGetLastError();
     }
     if (a.M == 0 || schedule != ZGL_TRACE_PERSISTENT || counter == nullptr) {

@@ -13,6 +13,7 @@
 #include "path_trace.cuh"
 #include "scene.h"
 #include "shading.cuh"
+#include "staged.h"
 #include "zgl_internal.h"
 
 struct zgl_integrator {
@@ -26,8 +27,9 @@ struct zgl_integrator {
     float* d_film = nullptr;    // light / triple: RGB sum, filmW * filmH * 3 (the r32f 3W x H film)
     float samplePerPixel = 0.0f;
     int32_t blocks = 0, loops = 1;
-    float* d_passes = nullptr;  // path tracer, several passes per launch: per-pass radiance
+    float* d_passes = nullptr;  // path tracer: per-pass radiance of one call
     size_t passesCap = 0;       // floats allocated in d_passes
+    zgl::StagedPool pool;       // path tracer, where it runs staged
 };
 
 #define ZGL_RENDER_NS plain
@@ -67,6 +69,39 @@ bool is_device_memory(const void* p) {
         return false;
     }
     return attr.type == cudaMemoryTypeDevice || attr.type == cudaMemoryTypeManaged;
+}
+
+// Whether a call of n passes runs staged (with room for it in the pool).
+// Trees of the long-ray kernels stay with them: in their 16x8 blocks the
+// lane-group walk (traverse.cuh: traverse_group) takes threadIdx.x for the
+// lane, so a few pixels a pass (4 of 2M on the benchmark's city) get another
+// value than the reference loop's, and frames are to stay as they are.
+bool runs_staged(const zgl_integrator* it, int64_t n) {
+    const zgl_scene* sc = it->scene;
+    const int64_t paths = (int64_t)sc->filmW * sc->filmH * n;
+    return it->pool.arena != nullptr && !long_ray_scene(sc) && it->passesCap >= (size_t)(3 * paths) && staged_pays(sc->view(), paths);
+}
+
+// Passes [curSample, curSample + n) of the path tracer, staged.  `f0` is the
+// first pass's freeCounter.
+void staged_passes(zgl_integrator* it, int32_t f0, int32_t n, cudaStream_t st) {
+    const zgl_scene* sc = it->scene;
+    const zgl_integrator_params& p = it->params;
+    StagedJob job{};
+    job.sc = sc->view();
+    job.maxDepth = p.max_depth;
+    job.rr = p.russian_roulette;
+    job.rrStart = p.rr_start_depth;
+    job.sampleLight = p.sample_light;
+    job.uniformSel = p.light_env_uniform_sample;
+    job.portion = p.light_portion;
+    job.full = sc->fullMaterials;
+    job.first = it->curSample;
+    job.n = n;
+    job.counter0 = f0 - it->curSample;
+    job.out = it->d_passes;
+    ZGL_CUDA(launch_staged(it->pool, job, st));
+    ZGL_CUDA(plain::launch_accumulate_passes(sc, it->curSample, n, it->d_passes, it->d_frame, st));
 }
 
 }  // namespace
@@ -119,6 +154,21 @@ zgl_status zgl_integrator_create(zgl_scene* scene, int32_t kind, const zgl_integ
         e = cudaMalloc(&it->d_film, sizeof(float) * 3 * npix);
         if (e == cudaSuccess) e = cudaMemset(it->d_film, 0, sizeof(float) * 3 * npix);
     }
+    if (e == cudaSuccess && kind == ZGL_INTEGRATOR_PATH && !long_ray_scene(scene) &&
+        staged_covers(scene->view(), p.max_depth) &&
+        staged_pays(scene->view(), (int64_t)npix)) {
+        // room for one pass now, so that a pass allocates nothing; without it
+        // the one-kernel path tracer runs
+        it->passesCap = 3 * npix;
+        e = cudaMalloc(&it->d_passes, sizeof(float) * it->passesCap);
+        if (e != cudaSuccess || !staged_alloc(it->pool, staged_paths(scene->filmW, scene->filmH, 1))) {
+            cudaGetLastError();
+            if (it->d_passes) cudaFree(it->d_passes);
+            it->d_passes = nullptr;
+            it->passesCap = 0;
+            e = cudaSuccess;
+        }
+    }
     if (e != cudaSuccess) {
         if (it->d_frame) cudaFree(it->d_frame);
         if (it->d_film) cudaFree(it->d_film);
@@ -141,8 +191,12 @@ zgl_status zgl_integrator_render_pass(zgl_integrator* it, void* stream) {
             it->finished = true;
             return ZGL_OK;
         }
-        const auto pass = long_ray_scene(sc) ? long_rays::launch_path_pass : plain::launch_path_pass;
-        ZGL_CUDA(pass(sc, it->params, it->curSample, it->freeCounter, it->d_frame, st));
+        if (runs_staged(it, 1)) {
+            staged_passes(it, it->freeCounter, 1, st);
+        } else {
+            const auto pass = long_ray_scene(sc) ? long_rays::launch_path_pass : plain::launch_path_pass;
+            ZGL_CUDA(pass(sc, it->params, it->curSample, it->freeCounter, it->d_frame, st));
+        }
     } else if (it->kind == ZGL_INTEGRATOR_LIGHT) {
         if (it->params.finite_sample && it->samplePerPixel > (float)it->params.max_sample) {
             it->finished = true;
@@ -192,8 +246,16 @@ zgl_status zgl_integrator_render_passes(zgl_integrator* it, int32_t passes, void
             ZGL_CUDA(cudaMalloc(&it->d_passes, sizeof(float) * need));
             it->passesCap = need;
         }
-        const auto passes = long_ray_scene(sc) ? long_rays::launch_path_passes : plain::launch_path_passes;
-        ZGL_CUDA(passes(sc, it->params, it->curSample, f0, n, it->d_passes, it->d_frame, (cudaStream_t)stream));
+        const int64_t paths = std::min(staged_paths(sc->filmW, sc->filmH, n), kStagedPaths);
+        if (!long_ray_scene(sc) && staged_covers(sc->view(), it->params.max_depth) &&
+            staged_pays(sc->view(), (int64_t)sc->filmW * sc->filmH * n) && it->pool.paths < paths)
+            staged_alloc(it->pool, paths);  // without the memory: the smaller pool, or one kernel
+        if (runs_staged(it, n)) {
+            staged_passes(it, f0, n, (cudaStream_t)stream);
+        } else {
+            const auto passes = long_ray_scene(sc) ? long_rays::launch_path_passes : plain::launch_path_passes;
+            ZGL_CUDA(passes(sc, it->params, it->curSample, f0, n, it->d_passes, it->d_frame, (cudaStream_t)stream));
+        }
         it->curSample += n;
     }
     if (n < passes) it->finished = true;
@@ -312,6 +374,7 @@ zgl_status zgl_integrator_destroy(zgl_integrator* it) {
     if (it->d_frame) cudaFree(it->d_frame);
     if (it->d_film) cudaFree(it->d_film);
     if (it->d_passes) cudaFree(it->d_passes);
+    staged_free(it->pool);
     delete it;
     ZGL_API_END
 }

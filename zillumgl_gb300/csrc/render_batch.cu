@@ -29,8 +29,10 @@
 
 #define ZGL_INLINE_TRACE 1
 #include "batch_flat.h"
+#include "path_step.cuh"
 #include "scene.h"
 #include "shading.cuh"
+#include "staged.h"
 #include "zgl_internal.h"
 
 namespace zgl {
@@ -38,14 +40,9 @@ namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
 
-struct BatchPathParams {
-    int32_t maxDepth, rr, rrStart, sampleLight, uniformSel;
-    float portion;
-};
-
 struct BatchRequest {
     DeviceScene sc;
-    BatchPathParams pp;
+    PathParams pp;
     int32_t spp;
     float4* frame;
     float* scratch;    // per-sample radiance of the current chunk, [sample - j0][npix][3]
@@ -54,6 +51,7 @@ struct BatchRequest {
     int32_t tilesX;    // 8x4 pixel tiles per film row
     int32_t perSample; // items per sample (whole tiles)
     int32_t j1;        // samples [j0, j1) of this request in the launch
+    bool full;         // metal-workflow or dielectric materials
 };
 
 constexpr int kMaxReqPerLaunch = 64;
@@ -71,36 +69,6 @@ struct BatchLaunch {
     const uint32_t* rows;   // Sobol rows: 256 values per sample index
 };
 static_assert(sizeof(BatchLaunch) <= 32000, "kernel parameter block too large");
-
-template <class Vis>
-__device__ __forceinline__ LiSample sampleLightAndEnvB(const DeviceScene& sc, const BatchPathParams& pp, v3 x,
-                                                       float ud, float u0, float u1, float u2, float u3,
-                                                       const Vis& vis) {
-    float pdfSampleLight = 0.0f;  // light.glsl:221-235
-    if (sc.nLight > 0) pdfSampleLight = pdfSampleLightSel(sc, pp.uniformSel, pp.portion);
-    bool sampleLight = ud < pdfSampleLight;
-    float pdfSelect = sampleLight ? pdfSampleLight : 1.0f - pdfSampleLight;
-    LiSample s;
-    if (sampleLight) {
-        int id = lightSampleOne(sc, mk2(u0, u1));
-        s = lightSampleLiV(sc, id, x, mk2(u2, u3), vis);
-    } else {
-        s = envSampleLiV(sc, x, u0, u1, u2, u3, vis);
-    }
-    s.coef = s.coef / pdfSelect;
-    s.pdf *= pdfSelect;
-    return s;
-}
-
-struct PathState {
-    Ray ray;        // pending ray
-    v3 result, throughput;
-    v3 wo, pos;     // vertex being left (valid after the first bounce)
-    v3 bsdfOverPdf; // bsdf / pdf of the last sample (Russian roulette)
-    float bsdfPdf;
-    int32_t bounce; // 0 = camera ray pending
-    bool delta;
-};
 
 __device__ __forceinline__ uint32_t sample_offset_dev(int32_t spp) {
     int32_t off = (int32_t)((uint32_t)spp * 256u);
@@ -130,132 +98,12 @@ __device__ __forceinline__ void start_sample(const BatchRequest& rq, const Batch
     st.bounce = 0;
 }
 
-// The light sample of a vertex whose occlusion test is left to a later
-// trace: the shadow ray and the contribution the sample makes if nothing
-// blocks it.
-struct PendingShadow {
-    v3 o, d, C;
-    float tmax;
-    bool pending;
-};
-
-// Visibility source that records the shadow ray instead of tracing it and
-// answers "not occluded"; the contribution is added after the trace.
-struct DeferVis {
-    PendingShadow* ps;
-    __device__ __forceinline__ bool operator()(const DeviceScene&, const Ray& r, float dist) const {
-        ps->o = r.ori;
-        ps->d = r.dir;
-        ps->tmax = dist;
-        return false;
-    }
-};
-
-// One step of pathIntegTrace after the pending ray has been traced (closest
-// hit `id` at `dist`): account for what it hits and, if the path continues,
-// shade the new vertex (light sample + BSDF sample) to produce the next
-// pending ray.  Returns false when the path ends.  DEFER: the light sample's
-// occlusion test is recorded in `ps` for a later trace instead of run here.
-template <bool FULL, bool DEFER>
-__device__ __forceinline__ bool path_step_hit(const BatchRequest& rq, Sampler& g, PathState& st, int id, float dist,
-                                              PendingShadow* ps) {
-    const DeviceScene& sc = rq.sc;
-    const BatchPathParams& pp = rq.pp;
-    v3 hitPos = rayPoint(st.ray, dist);
-    if (st.bounce == 0) {
-        // primary hit (path_integ_naive.glsl:37-44)
-        if (id == -1) {
-            st.result = envLe(sc, st.ray.dir);
-            return false;
-        }
-        if (id - sc.objPrimCount >= 0) {
-            st.result = lightLe(sc, id - sc.objPrimCount, hitPos, -st.ray.dir);
-            return false;
-        }
-        st.wo = -st.ray.dir;
-    } else {
-        // extension hit of bounce st.bounce (path_integ_naive.glsl:97-133)
-        v3 wi = st.ray.dir;
-        int lightId = id - sc.objPrimCount;
-        if (id == -1) {
-            v3 radiance = envLe(sc, wi);
-            float weight = 1.0f;
-            if (pp.sampleLight && !st.delta) {
-                float envPdf = envPdfLi(sc, wi) * (pp.uniformSel ? (1.0f - pp.portion)
-                                                                 : sc.envSum / (sc.lightSum + sc.envSum));
-                weight = (envPdf <= 0.0f) ? 0.0f : biHeuristic(st.bsdfPdf, envPdf);
-            }
-            st.result = st.result + radiance * st.throughput * weight;
-            return false;
-        }
-        if (lightId >= 0) {
-            v3 radiance = lightLe(sc, lightId, hitPos, -wi);
-            float weight = 1.0f;
-            if (pp.sampleLight && !st.delta) {
-                float snd = pp.uniformSel ? pp.portion : sc.lightSum / (sc.lightSum + sc.envSum);
-                float lightPdf = lightPdfLi(sc, lightId, st.pos, hitPos) * (lightPdfSampleOne(sc, lightId) * snd);
-                weight = (lightPdf <= 0.0f) ? 0.0f : biHeuristic(st.bsdfPdf, lightPdf);
-            }
-            st.result = st.result + radiance * st.throughput * weight;
-            return false;
-        }
-        if (pp.rr && st.bounce >= pp.rrStart) {
-            float continueProb = zmin(maxComponent(st.bsdfOverPdf), 0.95f);
-            if (sample1D(g) >= continueProb) return false;
-            st.throughput = st.throughput / continueProb;
-        }
-        st.wo = -wi;
-    }
-    // next bounce at the new vertex
-    st.bounce++;
-    if (st.bounce > pp.maxDepth) return false;
-    st.pos = hitPos;
-    TriShade tri = loadTri(sc, id);
-    Surface surf = surfaceInfo(tri, hitPos);
-    int matId = tri.matTex & 0x0000ffff;
-    uint32_t matType = loadMaterialType(sc, matId);
-    if (matType != kDielectric && matType != kThinDielectric && dot(surf.ns, st.wo) < 0.0f) {
-        surf.ns = -surf.ns;
-        surf.ng = -surf.ng;
-    }
-    BSDFParam mp = loadMaterial<FULL>(sc, matType, tri.matTex, id, surf);
-    if (pp.sampleLight) {
-        float ud = sample1D(g);
-        float u0 = sample1D(g), u1 = sample1D(g), u2 = sample1D(g),
-              u3 = sample1D(g);
-        LiSample ls;
-        if (DEFER) ls = sampleLightAndEnvB(sc, pp, hitPos, ud, u0, u1, u2, u3, DeferVis{ps});
-        else ls = sampleLightAndEnvB(sc, pp, hitPos, ud, u0, u1, u2, u3, TraceVis{});
-        if (ls.pdf > 0.0f) {
-            v3 f = materialBSDF<FULL>(matType, mp, st.wo, ls.wi, surf.ns);
-            float fpdf = materialPdf<FULL>(matType, mp, st.wo, ls.wi, surf.ns);
-            float weight = biHeuristic(ls.pdf, fpdf);
-            const v3 C = f * st.throughput * satDot(surf.ns, ls.wi) * ls.coef * weight;
-            if (DEFER) {
-                ps->C = C;
-                ps->pending = true;
-            } else {
-                st.result = st.result + C;
-            }
-        }
-    }
-    float b0 = sample1D(g), b1 = sample1D(g), b2 = sample1D(g);
-    BSDFSample bs = materialSample<FULL>(matType, mp, surf.ns, st.wo, mk3(b0, b1, b2), g);
-    st.delta = (bs.flag == kSpecRefl || bs.flag == kSpecTrans);
-    if (bs.pdf < 1e-8f) return false;
-    st.throughput = st.throughput * (bs.bsdf / bs.pdf * (st.delta ? 1.0f : absDot(surf.ns, bs.wi)));
-    st.bsdfPdf = bs.pdf;
-    st.bsdfOverPdf = bs.bsdf / bs.pdf;
-    st.ray = rayOffseted(hitPos, bs.wi);
-    return true;
-}
-
 // One step with the pending ray traced here.
 template <bool FULL>
 __device__ __forceinline__ bool path_step(const BatchRequest& rq, Sampler& g, PathState& st) {
     float dist;
     const int id = bvhHit(rq.sc, st.ray, dist);
-    return path_step_hit<FULL, false>(rq, g, st, id, dist, nullptr);
+    return path_step_hit<FULL, false>(rq.sc, rq.pp, g, st, id, dist, nullptr);
 }
 
 __device__ __forceinline__ int find_request(const BatchLaunch& L, int64_t item) {
@@ -492,7 +340,7 @@ __global__ void __launch_bounds__(kQueueBlock, 4) batch_queue_kernel(const __gri
                 if (!sOcc[tid]) st.result = st.result + ps.C;
                 ps.pending = false;
             }
-            if (!path_step_hit<FULL, true>(rq, g, st, cId[tid], cT[tid], &ps)) {
+            if (!path_step_hit<FULL, true>(rq.sc, rq.pp, g, st, cId[tid], cT[tid], &ps)) {
                 float* o = rq.scratch + 3 * ((size_t)(js - L.j0) * rq.npix + (size_t)py * rq.sc.filmW + px);
                 o[0] = st.result.x;
                 o[1] = st.result.y;
@@ -594,6 +442,7 @@ struct zgl_batch {
     uint32_t* d_rows = nullptr;     // maxSpp x 256 Sobol values
     float* d_scratch = nullptr;     // per request: min(spp, chunkLen) x npix x 3
     unsigned long long* d_counters = nullptr;
+    zgl::StagedPool pool;           // the flat schedule's, when every request runs staged
     int32_t nchunks_cap = 0;
     zgl_batch_config cfg{};
     cudaStream_t stream = nullptr;
@@ -615,6 +464,7 @@ void batch_free(zgl_batch* b) {
     if (b->d_rows) cudaFree(b->d_rows);
     if (b->d_scratch) cudaFree(b->d_scratch);
     if (b->d_counters) cudaFree(b->d_counters);
+    staged_free(b->pool);
     delete b;
 }
 
@@ -636,6 +486,11 @@ void check_config(const zgl_batch_config& c) {
     if (c.schedule != ZGL_BATCH_DEFAULT && c.schedule != ZGL_BATCH_FLAT && c.schedule != ZGL_BATCH_PERSISTENT &&
         c.schedule != ZGL_BATCH_QUEUE)
         fail(ZGL_ERR_INVALID_ARG, "batch: unknown schedule %d", c.schedule);
+}
+
+// Whether n samples of a request run on the staged path tracer.
+bool runs_staged(const BatchRequest& q, int n) {
+    return staged_covers(q.sc, q.pp.maxDepth) && staged_pays(q.sc, (int64_t)q.npix * n);
 }
 
 // Enqueues the whole render on `st`: frame clears, then per chunk of sample
@@ -691,11 +546,30 @@ void enqueue_render(zgl_batch* b, const zgl_batch_config& c, cudaStream_t st, in
                 ZGL_CUDA(cudaMemsetAsync(L.counter, 0, sizeof(unsigned long long), st));
                 ZGL_CUDA(launch_batch_queue(L, b->fullMaterials, st));
             } else {
+                // requests with paths enough run staged, one after the other;
+                // the rest share one launch of the one-kernel path tracer
                 FlatLaunch F;
                 std::memset(&F, 0, sizeof(F));
                 int64_t bb = 0;
                 for (int i = 0; i < L.nreq; i++) {
                     const BatchRequest& q = L.req[i];
+                    if (b->pool.arena && runs_staged(q, q.j1 - j0)) {
+                        StagedJob job{};
+                        job.sc = q.sc;
+                        job.maxDepth = q.pp.maxDepth;
+                        job.rr = q.pp.rr;
+                        job.rrStart = q.pp.rrStart;
+                        job.sampleLight = q.pp.sampleLight;
+                        job.uniformSel = q.pp.uniformSel;
+                        job.portion = q.pp.portion;
+                        job.full = q.full;
+                        job.first = j0;
+                        job.n = q.j1 - j0;
+                        job.counter0 = 1;
+                        job.out = q.scratch;
+                        ZGL_CUDA(launch_staged(b->pool, job, st));
+                        continue;
+                    }
                     FlatRequest& f = F.req[F.nreq++];
                     f.sc = q.sc;
                     f.maxDepth = q.pp.maxDepth;
@@ -709,13 +583,13 @@ void enqueue_render(zgl_batch* b, const zgl_batch_config& c, cudaStream_t st, in
                     f.tilesY = (q.sc.filmH + 7) / 8;
                     f.j1 = q.j1;
                     f.blockBase = bb;
+                    F.full = F.full || q.full;
                     bb += (int64_t)f.tilesX * f.tilesY * (q.j1 - j0);
                 }
                 F.nblocks = bb;
                 F.j0 = j0;
                 F.rows = b->d_rows;
                 F.mats = b->d_mats;
-                F.full = b->fullMaterials;
                 if (bb > 0x7fffffff) fail(ZGL_ERR_INVALID_ARG, "batch: too many tiles in one launch");
                 ZGL_CUDA(launch_batch_flat(F, st));
             }
@@ -768,11 +642,12 @@ zgl_status zgl_batch_create(const zgl_render_request* requests, int32_t n, const
                 fail(ZGL_ERR_INVALID_ARG, "zgl_batch_create: request %d has invalid parameters", i);
             BatchRequest q{};
             q.sc = r.scene->view();
-            q.pp = BatchPathParams{p.max_depth, p.russian_roulette, p.rr_start_depth, p.sample_light,
+            q.pp = PathParams{p.max_depth, p.russian_roulette, p.rr_start_depth, p.sample_light,
                                    p.light_env_uniform_sample, p.light_portion};
             q.spp = r.spp;
             q.frame = reinterpret_cast<float4*>(r.frame);
             q.npix = r.scene->filmW * r.scene->filmH;
+            q.full = r.scene->fullMaterials;
             q.tilesX = (r.scene->filmW + 7) / 8;
             q.perSample = q.tilesX * ((r.scene->filmH + 3) / 4) * 32;
             q.itemBase = base;
@@ -819,6 +694,13 @@ zgl_status zgl_batch_create(const zgl_render_request* requests, int32_t n, const
             q.scratch = b->d_scratch + off;
             off += (size_t)std::min(b->chunkLen, q.spp) * (size_t)q.npix * 3;
         }
+        // the staged path tracer's pool, for the largest request of a launch
+        int64_t paths = 0;
+        for (const auto& q : b->req) {
+            const int n = std::min(b->chunkLen, q.spp);
+            if (runs_staged(q, n)) paths = std::max(paths, staged_paths(q.sc.filmW, q.sc.filmH, n));
+        }
+        if (paths > 0) staged_alloc(b->pool, paths);
         const int nChunks = (b->maxSpp + b->chunkLen - 1) / b->chunkLen;
         b->nchunks_cap = nChunks * ((n + kMaxReqPerLaunch - 1) / kMaxReqPerLaunch);
         ZGL_CUDA(cudaMalloc(&b->d_counters, sizeof(unsigned long long) * (size_t)b->nchunks_cap));

@@ -28,6 +28,7 @@
 #include "bsdf_grad.cuh"
 #include "path_trace.cuh"
 #include "scene.h"
+#include "staged.h"
 #include "zgl_internal.h"
 
 struct zgl_diff {
@@ -41,6 +42,7 @@ struct zgl_diff {
     int2* d_hits = nullptr;       // kCastDepth * spp * npix (primitive id, distance bits)
     uint32_t* d_vis = nullptr;    // spp * npix light-sample occlusion bits
     bool castsValid = false;
+    zgl::StagedPool pool;         // the forward's, where it runs staged
     float* d_dimage = nullptr;    // npix * 3, zgl_diff_step_l2's dloss/dimage
     int32_t* d_lightInst = nullptr;  // per light triangle: instance index
     float* d_values = nullptr;       // current parameter values
@@ -494,6 +496,8 @@ zgl_status zgl_diff_create(zgl_scene* scene, const zgl_integrator_params* params
             ZGL_CUDA(cudaMalloc(&d->d_hits, sizeof(int2) * kCastDepth * paths));
             ZGL_CUDA(cudaMalloc(&d->d_vis, sizeof(uint32_t) * paths));
         }
+        if (staged_covers(scene->view(), d->params.max_depth) && staged_pays(scene->view(), (int64_t)paths))
+            staged_alloc(d->pool, staged_paths(scene->filmW, scene->filmH, spp));
         std::vector<int32_t> inst((size_t)std::max(scene->nLight, 1), 0);
         for (int k = 0; k < d->ninst; k++)
             for (uint32_t t = d->lightFirst[(size_t)k]; t < d->lightFirst[(size_t)k + 1]; t++) inst[t] = k;
@@ -515,6 +519,7 @@ zgl_status zgl_diff_create(zgl_scene* scene, const zgl_integrator_params* params
         if (d->d_vis) cudaFree(d->d_vis);
         if (d->d_lightInst) cudaFree(d->d_lightInst);
         if (d->d_values) cudaFree(d->d_values);
+        staged_free(d->pool);
         delete d;
         throw;
     }
@@ -563,7 +568,26 @@ zgl_status zgl_diff_forward(zgl_diff* d, float* image, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
     int tilesX = (s->filmW + kTileX - 1) / kTileX, tilesY = (s->filmH + kTileY - 1) / kTileY;
     dim3 grid((unsigned)(tilesX * tilesY), (unsigned)d->spp);
-    if (s->fullMaterials)
+    if (d->pool.arena) {
+        const zgl_integrator_params& p = d->params;
+        StagedJob job{};
+        job.sc = s->view();
+        job.maxDepth = p.max_depth;
+        job.rr = p.russian_roulette;
+        job.rrStart = p.rr_start_depth;
+        job.sampleLight = p.sample_light;
+        job.uniformSel = p.light_env_uniform_sample;
+        job.portion = p.light_portion;
+        job.full = s->fullMaterials;
+        job.first = 0;
+        job.n = d->spp;
+        job.counter0 = 1;
+        job.out = d->d_samples;
+        job.hits = d->d_hits;
+        job.castDepth = kCastDepth;
+        job.vis = d->d_vis;
+        ZGL_CUDA(launch_staged(d->pool, job, st));
+    } else if (s->fullMaterials)
         diff_forward_kernel<true><<<grid, dim3(kTileX, kTileY), 0, st>>>(s->view(), path_params(d->params), tilesX,
                                                                          d->spp, d->d_samples, d->d_hits, d->d_vis);
     else
@@ -633,6 +657,7 @@ zgl_status zgl_diff_destroy(zgl_diff* d) {
     if (d->d_dimage) cudaFree(d->d_dimage);
     if (d->d_lightInst) cudaFree(d->d_lightInst);
     if (d->d_values) cudaFree(d->d_values);
+    staged_free(d->pool);
     delete d;
     ZGL_API_END
 }

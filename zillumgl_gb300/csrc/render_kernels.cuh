@@ -590,6 +590,13 @@ cudaError_t launch_path_pass(const zgl_scene* s, const zgl_integrator_params& p,
     return cudaGetLastError();
 }
 
+cudaError_t launch_accumulate_passes(const zgl_scene* s, int32_t c0, int32_t n, const float* scratch, float4* frame,
+                                     cudaStream_t st) {
+    const int64_t npix = (int64_t)s->filmW * s->filmH;
+    accumulate_passes_kernel<<<(unsigned)((npix + 255) / 256), 256, 0, st>>>(scratch, npix, c0, n, frame);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_path_passes(const zgl_scene* s, const zgl_integrator_params& p, int32_t c0, int32_t f0, int32_t n,
                                float* scratch, float4* frame, cudaStream_t st) {
     PathParams pp{p.max_depth, p.russian_roulette, p.rr_start_depth, p.sample_light, p.light_env_uniform_sample,
@@ -602,9 +609,7 @@ cudaError_t launch_path_passes(const zgl_scene* s, const zgl_integrator_params& 
         path_passes_kernel<false><<<grid, block, 0, st>>>(s->view(), pp, c0, f0, scratch);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    const int64_t npix = (int64_t)s->filmW * s->filmH;
-    accumulate_passes_kernel<<<(unsigned)((npix + 255) / 256), 256, 0, st>>>(scratch, npix, c0, n, frame);
-    return cudaGetLastError();
+    return launch_accumulate_passes(s, c0, n, scratch, frame, st);
 }
 
 #if !ZGL_LONG_RAYS

@@ -24,6 +24,8 @@ namespace zgl {
 namespace plain {
 ZGL_RENDER_LAUNCHERS
 cudaError_t launch_film_to_frame(const float* film, float4* out, int64_t n, cudaStream_t st);
+cudaError_t launch_accumulate_passes(const zgl_scene* s, int32_t c0, int32_t n, const float* scratch, float4* frame,
+                                     cudaStream_t st);
 }  // namespace plain
 namespace long_rays {
 ZGL_RENDER_LAUNCHERS

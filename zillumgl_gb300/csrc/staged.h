@@ -1,0 +1,77 @@
+// staged.h — the staged path tracer (staged.cu): a path's ray casts and its
+// shading in separate kernels, for every caller that renders whole samples of
+// one scene (progressive passes, several passes at once, the batched
+// renderer, the differentiable forward pass).
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+#include "device_scene.h"
+
+namespace zgl {
+
+// Paths in flight at most: two float4 x 4 + uint2 states, a hit and a shadow
+// ray each (about 230 B), 480 MB in all; a 1080p pass fits.
+constexpr int64_t kStagedPaths = 1 << 21;
+// Depth from which the one-kernel path tracer runs instead: the staged one
+// launches two kernels per bounce whether or not a path gets there.
+constexpr int32_t kStagedMaxDepth = 24;
+// Sample indices whose Sobol rows fit the pool's table.
+constexpr int32_t kStagedRows = 256;
+
+// Device memory of a staged render of up to `paths` paths at a time.
+struct StagedPool {
+    void* arena = nullptr;
+    int64_t paths = 0;
+    float4 *org[2], *dir[2], *thr[2], *pos[2];
+    uint2* rng[2];
+    int2* hit;
+    float4 *sorg, *sdir, *scon;
+    uint32_t* counts;  // per step: paths, shadow rays
+    uint32_t* rows;    // kStagedRows x 256
+};
+
+// Pool for renders of `total` paths in place of what `p` holds; false without
+// the memory (`p` is then as it was, and the caller keeps to one kernel or to
+// the smaller pool).
+bool staged_alloc(StagedPool& p, int64_t total);
+void staged_free(StagedPool& p);
+
+// Samples s in [first, first + n) of every pixel of a scene, `maxDepth` at
+// most kStagedMaxDepth.  Sample s uses Sobol row sample_offset(s) and
+// freeCounter s + counter0; its radiance goes to out[(s - first) * npix +
+// pix][3].  With `hits`, the first `castDepth` closest hits of each path go to
+// hits[(k * n + s - first) * npix + pix] and the occlusion answers of its
+// first 32 light samples to vis[(s - first) * npix + pix].
+struct StagedJob {
+    DeviceScene sc;
+    int32_t maxDepth, rr, rrStart, sampleLight, uniformSel;
+    float portion;
+    bool full;  // metal-workflow or dielectric materials
+    int32_t first, n, counter0;
+    float* out;
+    int2* hits;
+    int32_t castDepth;
+    uint32_t* vis;
+};
+cudaError_t launch_staged(const StagedPool& pool, const StagedJob& job, cudaStream_t st);
+
+// Whether a scene and depth run staged.
+inline bool staged_covers(const DeviceScene& sc, int32_t maxDepth) {
+    return sc.accel.wide != nullptr && maxDepth >= 0 && maxDepth <= kStagedMaxDepth;
+}
+// Whether it is the faster way for a call of `paths` paths.  Two launches a
+// bounce have a latency that few paths do not fill: on a 2k-triangle box 65k
+// paths take 0.47 ms staged and 0.40 in one kernel, 147k 0.59 and 0.73; on
+// 100k triangles 16k paths take 0.59 and 0.69, 65k 0.68 and 0.75.
+inline bool staged_pays(const DeviceScene& sc, int64_t paths) {
+    return paths >= 98304 || (sc.accel.M >= 16384 && paths >= 32768);
+}
+// Paths of n samples per pixel, film edges padded to whole tiles.
+inline int64_t staged_paths(int32_t filmW, int32_t filmH, int64_t n) {
+    return (int64_t)((filmW + 7) / 8) * ((filmH + 3) / 4) * 32 * n;
+}
+
+}  // namespace zgl

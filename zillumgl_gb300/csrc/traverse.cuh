@@ -110,18 +110,17 @@ __device__ __forceinline__ bool box_hit(const float4 lo, const float4 hi, const 
 
 // intersectTriangle with precomputed a, ab = b - a, ac = c - a, in the three
 // float4 of a traversal triangle (a.xyz ab.x | ab.yz ac.xy | ac.z ...).
-__device__ __forceinline__ bool tri_test(const float4 t0, const float4 t1, const float4 t2, const TraceRay& r,
-                                         float& t) {
+__device__ __forceinline__ bool tri_test(const float4 t0, const float4 t1, const float4 t2, const float3 o,
+                                         const float3 d, float& t) {
     const float abx = t0.w, aby = t1.x, abz = t1.y;
     const float acx = t1.z, acy = t1.w, acz = t2.x;
-    const float3 d = r.d;
     // p = cross(d, ac); det = dot(ab, p)
     float px = d.y * acz - d.z * acy;
     float py = d.z * acx - d.x * acz;
     float pz = d.x * acy - d.y * acx;
     float det = abx * px + aby * py + abz * pz;
     if (fabsf(det) < 1e-6f) return false;
-    float aox = r.o.x - t0.x, aoy = r.o.y - t0.y, aoz = r.o.z - t0.z;
+    float aox = o.x - t0.x, aoy = o.y - t0.y, aoz = o.z - t0.z;
     if (det < 0.0f) {
         aox = -aox;
         aoy = -aoy;
@@ -143,7 +142,7 @@ __device__ __forceinline__ bool tri_test(const float4 t0, const float4 t1, const
 __device__ __forceinline__ bool tri_hit(const float4* __restrict__ tris, int prim,
                                         const TraceRay& r, float& t) {
     return tri_test(__ldg(tris + 3 * (size_t)prim), __ldg(tris + 3 * (size_t)prim + 1),
-                    __ldg(tris + 3 * (size_t)prim + 2), r, t);
+                    __ldg(tris + 3 * (size_t)prim + 2), r.o, r.d, t);
 }
 // bvhHit (ANY = false): returns the closest primitive or -1 and lowers `dist`.
 // bvhTest (ANY = true): returns 1 at the first t < dist, else 0.
@@ -379,24 +378,39 @@ __device__ __forceinline__ void traverse_warp(const DeviceAccel& a, const TraceR
         const int prim = __float_as_int(lo.w);
         const bool tri = geom && prim >= 0 && tri_hit(a.tris, prim, r, t);
         const int skip = max(__float_as_int(hi.w), j + 1);
-        const unsigned G = __ballot_sync(full, geom), T = __ballot_sync(full, tri);
-        // the path through the window: p only grows, so at most 32 steps
+        unsigned H = __ballot_sync(full, geom && !(tmin > dist)), T = __ballot_sync(full, tri);
+        // The path through the window, from miss to miss: the hits up to the
+        // next miss are consecutive entries, and only a triangle among them
+        // can change the distance.  p only grows.
         int p = 0;
         for (;;) {
-            const float tm = __shfl_sync(full, tmin, p);
-            const float tt = __shfl_sync(full, t, p);
-            const int pr = __shfl_sync(full, prim, p);
-            const int sk = __shfl_sync(full, skip, p);
-            const bool h = ((G >> p) & 1u) && !(tm > dist);
-            if (h && ((T >> p) & 1u) && tt < dist) {
-                closest = pr;
-                if (ANY) {
-                    k = M;
-                    return;
+            const unsigned from = 0xffffffffu << p;
+            const unsigned miss = ~H & from;
+            const int q = miss ? __ffs(miss) - 1 : 32;
+            const unsigned cand = T & H & from & (q < 32 ? (1u << q) - 1u : 0xffffffffu);
+            if (cand) {
+                const int c = __ffs(cand) - 1;
+                const float tt = __shfl_sync(full, t, c);
+                if (tt < dist) {
+                    closest = __shfl_sync(full, prim, c);
+                    if (ANY) {
+                        k = M;
+                        return;
+                    }
+                    dist = tt;
+                    H = __ballot_sync(full, geom && !(tmin > dist));
                 }
-                dist = tt;
+                T &= ~(1u << c);
+                p = c + 1;
+                if (p < 32) continue;
+                k += 32;
+                break;
             }
-            const int next = h ? k + p + 1 : max(sk, k + p + 1);  // the max holds by construction
+            if (q == 32) {
+                k += 32;
+                break;
+            }
+            const int next = __shfl_sync(full, skip, q);
             if (next >= M || next - k >= 32) {
                 k = next;
                 break;

@@ -59,9 +59,14 @@ namespace zgl {
 
 constexpr int kWideStack = 64;            // entries per thread (local memory)
 constexpr int kWideDone = (int)0x80000000;  // bottom of the stack
+// Nodes a ray of the rarer modes visits on its lane before its warp takes it
+// over on the face table: on meshes of small triangles, where P binds, such a
+// ray needs a few hundred; with large ones, tens of thousands.
+constexpr int kPadBudget = 4096;
 
-// Result of one wide traversal: `ok` false when the stack ran out (the caller
-// starts over with the reference loop).
+// Result of one wide traversal: `ok` false when the stack ran out or a ray of
+// the rarer modes outran kPadBudget nodes (triangles too large for P to
+// bind); the caller starts over with the reference loop.
 struct WideHit {
     int id;
     float dist;
@@ -117,7 +122,8 @@ __device__ __forceinline__ bool wide_covers(const TraceRay& r) {
 
 // boxHit on every ancestor of the triangle in leaf slot `slot` (the leaf
 // itself excluded), from the root down.
-static __device__ __noinline__ bool chain_accepts(const float4* dfs, int slot, TraceRay r) {
+static __device__ __noinline__ bool chain_accepts(const float4* dfs, int slot, float3 o, float3 d) {
+    const TraceRay r = make_trace_ray(o, d);
     int64_t k = 0;
     float4 lo = __ldg(dfs), hi = __ldg(dfs + 1);
     while (!(__float_as_uint(lo.w) & 0x80000000u)) {
@@ -191,8 +197,8 @@ struct WidePad {
 // entered, in visiting order.  PAD = false: rays of mode 3; PAD = true: every
 // other ray that wide_covers admits.
 template <bool PAD>
-__device__ __forceinline__ void wide_node(const float4* wide, const TraceRay& r, const WidePad& w, float dist,
-                                          int* stack, int& sp, int& cur) {
+__device__ __forceinline__ void wide_node(const float4* wide, const float3 o, const float3 inv, int face,
+                                          const WidePad& w, float dist, int* stack, int& sp, int& cur) {
     const float4* const n = wide + (size_t)(unsigned)cur * 4;
     unsigned u[8], v[8];
     load32(n, u);
@@ -201,33 +207,38 @@ __device__ __forceinline__ void wide_node(const float4* wide, const TraceRay& r,
     const float sx = __uint_as_float((u[3] << 23) & 0x7f800000u);
     const float sy = __uint_as_float((u[3] << 15) & 0x7f800000u);
     const float sz = __uint_as_float((u[3] << 7) & 0x7f800000u);
-    float4 nx, ny, nz, fx, fy, fz;
-    if (PAD) {
-        const float l2 = __uint_as_float((u[3] >> 1) & 0x7f800000u);
-        const float pad = l2 < 0.7f ? w.padA + w.padB * l2 : 1e30f;
-        const bool bx = w.ix < 0.0f, by = w.iy < 0.0f, bz = w.iz < 0.0f;
-        nx = slab4(bx ? v[1] : v[0], sx, gx, w.px ? -(r.o.x + pad) : -r.o.x, w.ix);
-        fx = slab4(bx ? v[0] : v[1], sx, gx, w.px ? -(r.o.x - pad) : -r.o.x, w.ix);
-        ny = slab4(by ? v[3] : v[2], sy, gy, w.py ? -(r.o.y + pad) : -r.o.y, w.iy);
-        fy = slab4(by ? v[2] : v[3], sy, gy, w.py ? -(r.o.y - pad) : -r.o.y, w.iy);
-        nz = slab4(bz ? v[5] : v[4], sz, gz, w.pz ? -(r.o.z + pad) : -r.o.z, w.iz);
-        fz = slab4(bz ? v[4] : v[5], sz, gz, w.pz ? -(r.o.z - pad) : -r.o.z, w.iz);
-    } else {
-        const bool bx = r.dinv.x < 0.0f, by = r.dinv.y < 0.0f, bz = r.dinv.z < 0.0f;
-        nx = slab4(bx ? v[1] : v[0], sx, gx, -r.o.x, r.dinv.x);
-        fx = slab4(bx ? v[0] : v[1], sx, gx, -r.o.x, r.dinv.x);
-        ny = slab4(by ? v[3] : v[2], sy, gy, -r.o.y, r.dinv.y);
-        fy = slab4(by ? v[2] : v[3], sy, gy, -r.o.y, r.dinv.y);
-        nz = slab4(bz ? v[5] : v[4], sz, gz, -r.o.z, r.dinv.z);
-        fz = slab4(bz ? v[4] : v[5], sz, gz, -r.o.z, r.dinv.z);
+    // one axis after the other, so that eight running bounds are live instead
+    // of 24 slab values (48 registers a thread)
+    float4 tn, tf;
+    {
+        const float inx = PAD ? w.ix : inv.x, iny = PAD ? w.iy : inv.y, inz = PAD ? w.iz : inv.z;
+        float pad = 0.0f;
+        if (PAD) {
+            const float l2 = __uint_as_float((u[3] >> 1) & 0x7f800000u);
+            pad = l2 < 0.7f ? w.padA + w.padB * l2 : 1e30f;
+        }
+        const bool bx = inx < 0.0f, by = iny < 0.0f, bz = inz < 0.0f;
+        const float xn = PAD && w.px ? -(o.x + pad) : -o.x, xf = PAD && w.px ? -(o.x - pad) : -o.x;
+        tn = slab4(bx ? v[1] : v[0], sx, gx, xn, inx);
+        tf = slab4(bx ? v[0] : v[1], sx, gx, xf, inx);
+        const float yn = PAD && w.py ? -(o.y + pad) : -o.y, yf = PAD && w.py ? -(o.y - pad) : -o.y;
+        float4 q = slab4(by ? v[3] : v[2], sy, gy, yn, iny);
+        tn = make_float4(fmaxf(tn.x, q.x), fmaxf(tn.y, q.y), fmaxf(tn.z, q.z), fmaxf(tn.w, q.w));
+        q = slab4(by ? v[2] : v[3], sy, gy, yf, iny);
+        tf = make_float4(fminf(tf.x, q.x), fminf(tf.y, q.y), fminf(tf.z, q.z), fminf(tf.w, q.w));
+        const float zn = PAD && w.pz ? -(o.z + pad) : -o.z, zf = PAD && w.pz ? -(o.z - pad) : -o.z;
+        q = slab4(bz ? v[5] : v[4], sz, gz, zn, inz);
+        tn = make_float4(max3f(tn.x, q.x, 0.0f), max3f(tn.y, q.y, 0.0f), max3f(tn.z, q.z, 0.0f), max3f(tn.w, q.w, 0.0f));
+        q = slab4(bz ? v[4] : v[5], sz, gz, zf, inz);
+        tf = make_float4(min3f(tf.x, q.x, dist), min3f(tf.y, q.y, dist), min3f(tf.z, q.z, dist), min3f(tf.w, q.w, dist));
     }
     // child reference, 0 (the root, never a child; also an empty slot) where missed
-    int r0 = fmaxf(max3f(nx.x, ny.x, nz.x), 0.0f) <= fminf(min3f(fx.x, fy.x, fz.x), dist) ? (int)u[4] : 0;
-    int r1 = fmaxf(max3f(nx.y, ny.y, nz.y), 0.0f) <= fminf(min3f(fx.y, fy.y, fz.y), dist) ? (int)u[5] : 0;
-    int r2 = fmaxf(max3f(nx.z, ny.z, nz.z), 0.0f) <= fminf(min3f(fx.z, fy.z, fz.z), dist) ? (int)u[6] : 0;
-    int r3 = fmaxf(max3f(nx.w, ny.w, nz.w), 0.0f) <= fminf(min3f(fx.w, fy.w, fz.w), dist) ? (int)u[7] : 0;
+    int r0 = tn.x <= tf.x ? (int)u[4] : 0;
+    int r1 = tn.y <= tf.y ? (int)u[5] : 0;
+    int r2 = tn.z <= tf.z ? (int)u[6] : 0;
+    int r3 = tn.w <= tf.w ? (int)u[7] : 0;
     // visiting order of the ray's face
-    const unsigned swaps = v[6] >> (3 * r.face);
+    const unsigned swaps = v[6] >> (3 * face);
     const int q0 = (swaps & 1u) ? r1 : r0, q1 = (swaps & 1u) ? r0 : r1;
     const int q2 = (swaps & 2u) ? r3 : r2, q3 = (swaps & 2u) ? r2 : r3;
     r0 = (swaps & 4u) ? q2 : q0;
@@ -241,26 +252,44 @@ __device__ __forceinline__ void wide_node(const float4* wide, const TraceRay& r,
     if (r0) { stack[sp++] = cur; cur = r0; }
 }
 
-// One triangle: whether the reference would take it at distance `dist`.
-template <bool PAD>
-__device__ __forceinline__ bool wide_leaf(const DeviceAccel& a, const TraceRay& r, int ref, float dist, float& t,
-                                          int& prim) {
-    const int slot = ~ref;
-    const float4* const tr = a.wtris + (size_t)(unsigned)slot * 4;
+// One triangle (rays of mode 3) against the reference: 0 not taken, 1 taken at
+// distance t, 2 taken if the ancestors' conditions hold, which the leaf's
+// slack leaves open.
+__device__ __forceinline__ int wide_leaf(const DeviceAccel& a, const float3 o, const float3 inv, const float3 d, int ref,
+                                         float dist, float& t, int& prim) {
+    const float4* const tr = a.wtris + (size_t)(unsigned)~ref * 4;
     unsigned u[8], v[8];
     load32(tr, u);
     load32(tr + 2, v);
     const auto f = [](unsigned x) { return __uint_as_float(x); };
     prim = (int)v[1];
     if (!tri_test(make_float4(f(u[0]), f(u[1]), f(u[2]), f(u[3])), make_float4(f(u[4]), f(u[5]), f(u[6]), f(u[7])),
-                  make_float4(f(v[0]), 0.0f, 0.0f, 0.0f), r, t) ||
+                  make_float4(f(v[0]), 0.0f, 0.0f, 0.0f), o, d, t) ||
         !(t < dist))
-        return false;
+        return 0;
+    TraceRay r;
+    r.o = o;
+    r.dinv = inv;
+    r.mode = 3;
     const float4 lo = make_float4(f(v[2]), f(v[3]), f(v[4]), 0.0f);
     const float4 hi = make_float4(f(v[5]), f(v[6]), f(v[7]), 0.0f);
     float tmin;
-    return (PAD ? box_hit(lo, hi, r, tmin) : box_hit_m<3>(lo, hi, r, tmin)) && !(tmin > dist) &&
-           (leaf_settles(a, lo, hi, r) || chain_accepts(a.dfs, slot, r));
+    if (!box_hit_m<3>(lo, hi, r, tmin) || tmin > dist) return 0;
+    return leaf_settles(a, lo, hi, r) ? 1 : 2;
+}
+
+// The same for any ray that wide_covers admits, the ancestors included.
+__device__ __forceinline__ bool wide_leaf_any_mode(const DeviceAccel& a, const TraceRay& r, int ref, float dist,
+                                                   float& t, int& prim) {
+    const int slot = ~ref;
+    const float4* const tr = a.wtris + (size_t)(unsigned)slot * 4;
+    const float4 t2 = __ldg(tr + 2), t3 = __ldg(tr + 3);
+    prim = __float_as_int(t2.y);
+    if (!tri_test(__ldg(tr), __ldg(tr + 1), t2, r.o, r.d, t) || !(t < dist)) return false;
+    const float4 lo = make_float4(t2.z, t2.w, t3.x, 0.0f), hi = make_float4(t3.y, t3.z, t3.w, 0.0f);
+    float tmin;
+    return box_hit(lo, hi, r, tmin) && !(tmin > dist) &&
+           (leaf_settles(a, lo, hi, r) || chain_accepts(a.dfs, slot, r.o, r.d));
 }
 
 // Closest hit (ANY = false) or any hit closer than `dist` of one ray.
@@ -269,17 +298,20 @@ __device__ __forceinline__ WideHit traverse_wide(const DeviceAccel& a, const Tra
     int stack[kWideStack];
     WidePad w;
     if (PAD) w.set(a, r);
-    int closest = -1, sp = 1, cur = 0;
+    int closest = -1, sp = 1, cur = 0, nodes = 0, budget = kPadBudget;
+    if (PAD && ((__float_as_uint(__ldg(reinterpret_cast<const float*>(a.wide) + 3)) >> 1) & 0x7f800000u) >=
+                   __float_as_uint(1.0f))
+        budget = kLongRayBudget;  // the root's l^2 passes 0.7
     stack[0] = kWideDone;
     for (;;) {
         while (cur >= 0) {
-            if (sp > kWideStack - 4) return WideHit{-1, dist, false};
-            wide_node<PAD>(a.wide, r, w, dist, stack, sp, cur);
+            if (sp > kWideStack - 4 || (PAD && ++nodes > budget)) return WideHit{-1, dist, false};
+            wide_node<PAD>(a.wide, r.o, r.dinv, r.face, w, dist, stack, sp, cur);
         }
         if (cur == kWideDone) break;
         float t;
         int prim;
-        if (wide_leaf<PAD>(a, r, cur, dist, t, prim)) {
+        if (wide_leaf_any_mode(a, r, cur, dist, t, prim)) {
             closest = prim;
             dist = t;
             if (ANY) break;
@@ -287,6 +319,229 @@ __device__ __forceinline__ WideHit traverse_wide(const DeviceAccel& a, const Tra
         cur = stack[--sp];
     }
     return WideHit{closest, dist, true};
+}
+
+// Rays that the wide tree's loop leaves out, marked by `want`: one per lane on
+// the wide tree, those it does not cover on the face table; those that outrun
+// kPadBudget nodes or kLongRayBudget entries there, or the stack, on the face
+// table with the whole warp.  Every lane calls.
+template <bool ANY>
+__device__ __forceinline__ bool lane_walk(const DeviceAccel& a, const TraceRay& r, float& dist, int& k, int& closest,
+                                          int budget) {
+    return budget > 0 && traverse_lane_m<ANY, false, 0>(a, r, dist, k, closest, budget);
+}
+template <class Io>
+static __device__ __noinline__ void wide_rest(DeviceAccel a, Io io, int i, bool want) {
+    const bool any = want && io.any(i);
+    const TraceRay r = make_trace_ray(want ? io.origin(i) : make_float3(0.0f, 0.0f, 0.0f),
+                                      want ? io.direction(i) : make_float3(0.0f, 0.0f, 1.0f));
+    float dist = want ? io.limit(i) : 0.0f;
+    int closest = -1;
+    bool done = !want;
+    int budget = kLongRayBudget;
+    if (want && wide_covers(r)) {
+        budget = 0;  // what stays unfinished here goes to the warp at once
+        WideHit h;
+        if (r.mode == 3) h = any ? traverse_wide<true, false>(a, r, dist) : traverse_wide<false, false>(a, r, dist);
+        else h = any ? traverse_wide<true, true>(a, r, dist) : traverse_wide<false, true>(a, r, dist);
+        if (h.ok) {
+            closest = h.id;
+            dist = h.dist;
+            done = true;
+        }
+    }
+    if (!__all_sync(0xffffffffu, done)) {
+        int k = 0, k2 = 0;
+        bool done1 = done || any, done2 = done || !any;
+        if (Io::kClosest) {
+            done1 = done1 || lane_walk<false>(a, r, dist, k, closest, budget);
+            finish_long_rays<false>(a, r, dist, k, closest, done1);
+        }
+        if (Io::kAny) {
+            done2 = done2 || lane_walk<true>(a, r, dist, k2, closest, budget);
+            finish_long_rays<true>(a, r, dist, k2, closest, done2);
+        }
+    }
+    if (want) io.store(i, closest, dist);
+}
+
+// Closest or any hit of n rays, one grid.  Io says what ray i is and takes its
+// result:
+//   kClosest, kAny    which queries occur
+//   any(i)            whether ray i asks for any hit
+//   origin, direction, limit(i)  the ray (limit: 1e8 or the any-hit distance)
+//   store(i, id, t)   id -1: nothing hit
+//   mark(i), marked(i)  sets ray i aside: a value its result never has
+//
+// Divergence is what this loop fights.  Rays of one warp visit between a few
+// and 400 nodes (mean 31 on the 4M soup's bounce rays, 4 triangles); one ray
+// per thread to the end kept 5.5 lanes busy and ran at 740 Mrays/s.  So
+//  * the grid is one wave of resident warps, each taking every nwarps-th group
+//    of 32 rays; lanes without a ray are refilled from the sequence once
+//    kRefill of them are idle (no counter in memory, so launches on other
+//    streams and in graphs stay independent).  256 consecutive rays per warp
+//    instead: 1083 Mrays/s against 1268 (its tails come once a launch);
+//  * a lane that reaches a triangle sets it aside and goes on with the nodes
+//    behind it (a later, larger distance only adds nodes; triangles are still
+//    tested in order).  The warp turns to the waiting triangles when fewer
+//    than kInner lanes have a node left (8 to 24 measured, flat at 16 to 20).
+// 64-byte nodes in two 32-byte loads: with 128-byte nodes of full floats in
+// eight 16-byte loads the L1 was 70% busy (a gather takes a cycle a lane) and
+// the same loop ran at 760 Mrays/s.  No call in the loop: 1268 -> 1601 Mrays/s
+// (see its end).  48 registers (20 blocks of 64 threads per SM) hide more
+// latency than 56 (1485) and 40 (1447).  4M soup, 4M bounce rays: 2.62 ms,
+// 7.35 before on the threaded tables; issue slots 61% and L1 66% busy, 19 of
+// 32 lanes active.
+constexpr int kWideBlock = 64;
+constexpr int kWideBlocksPerSM = 20;
+constexpr int64_t kWideMaxRays = int64_t(1) << 30;  // of one grid
+constexpr int kInner = 16;
+constexpr int kRefill = 8;
+
+// Rays per warp and round: 32, fewer when n does not give 32 to eight warps
+// per SM (see wide_blocks).
+__host__ __device__ __forceinline__ int wide_group(int64_t n, int sms) {
+    const int64_t g = (n + (int64_t)sms * 8 - 1) / ((int64_t)sms * 8);
+    return (int)(g < 1 ? 1 : g > 32 ? 32 : g);
+}
+// Blocks of kWideBlock threads for up to n rays (a kernel that gets a smaller
+// number from the device takes wide_group of that): one wave of resident
+// warps, and never fewer warps than wide_group counts on.  Rays
+// too few for eight warps of 32 per SM are spread thinner over eight warps per
+// SM, so that they do not wait for each other's branches (997 rays on 2048
+// triangles 76 -> 55 us, 5000 on 1M 237 -> 198 us with the whole launch).
+// Spreading over all resident warps is slower from 60,000 rays on (88 -> 101
+// us): full warps share their loads.
+inline unsigned wide_blocks(int64_t n, int sms) {
+    const int64_t warps = (int64_t)sms * kWideBlocksPerSM * (kWideBlock / 32);
+    const int64_t full = (n + 31) / 32 > (int64_t)sms * 8 ? (n + 31) / 32 : (int64_t)sms * 8;
+    int64_t used = full < warps ? full : warps;
+    used = n < used ? n : used;
+    return (unsigned)((used + kWideBlock / 32 - 1) / (kWideBlock / 32));
+}
+
+//
+// Every round of the loop makes progress: it takes new rays, steps a node, or
+// tests a triangle.  The node loop is left before
+// a step only for a waiting triangle, or when kRefill lanes are free or about
+// to be, which the next round refills.
+template <class Io>
+__device__ __forceinline__ void wide_trace(const DeviceAccel& a, const Io& io, int n, int group) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u;
+    // ray p of this warp's sequence is ray ((p / 32) * nwarps + warp) * 32 +
+    // p % 32; with fewer rays than that takes, the warp has `group` of them
+    const int warp = (int)(blockIdx.x * (kWideBlock / 32) + (threadIdx.x >> 5));
+    const int stride = (int)(gridDim.x * kWideBlock);
+    int taken = 0;
+    bool more = warp * group < n;
+    int stack[kWideStack];
+    stack[0] = kWideDone;
+    int ray = 0;
+    float3 o = make_float3(0.0f, 0.0f, 0.0f), inv = o;
+    const WidePad none{};
+    float dist = 0.0f;
+    int face = 0, closest = -1, sp = 1, cur = kWideDone, leaf = 0;
+    bool live = false, rest = false;  // rest: this lane set a ray aside
+    for (;;) {
+        // refill the lanes without a ray
+        const unsigned idle = __ballot_sync(full, !live);
+        if (idle == full && !more) break;
+        if (more && __popc(idle) >= kRefill) {
+            const int p = taken + __popc(idle & lt);
+            int mine;
+            if (group == 32) {
+                mine = (p >> 5) * stride + warp * 32 + (p & 31);
+                taken += __popc(idle);
+                more = (taken >> 5) * stride + warp * 32 + (taken & 31) < n;
+            } else {
+                mine = p < group ? warp * group + p : n;
+                more = false;
+            }
+            if (!live && mine < n) {
+                ray = mine;
+                const TraceRay r = make_trace_ray(io.origin(ray), io.direction(ray));
+                if (r.d.x == 0.0f && r.d.y == 0.0f && r.d.z == 0.0f) {
+                    // det is 0 for every triangle: nothing is hit (a BSDF
+                    // sample below the horizon leaves such a ray)
+                    io.store(ray, -1, io.limit(ray));
+                } else if (r.mode == 3 && wide_covers(r)) {
+                    o = r.o;
+                    inv = r.dinv;
+                    face = r.face;
+                    dist = io.limit(ray);
+                    closest = -1;
+                    sp = 1;
+                    cur = 0;
+                    live = true;
+                } else {
+                    io.mark(ray);
+                    rest = true;
+                }
+            }
+        }
+        // nodes, until few lanes have one and some wait with a triangle or
+        // could be refilled
+        for (;;) {
+            const unsigned inner = __ballot_sync(full, cur >= 0);
+            if (inner == 0u) break;
+            if (__popc(inner) < kInner &&
+                (__any_sync(full, leaf != 0) || (more && __popc(__ballot_sync(full, cur == kWideDone)) >= kRefill)))
+                break;
+            if (cur >= 0) {
+                if (sp > kWideStack - 4) {
+                    io.mark(ray);
+                    rest = true;
+                    live = false;
+                    cur = kWideDone;
+                    leaf = 0;
+                } else {
+                    wide_node<false>(a.wide, o, inv, face, none, dist, stack, sp, cur);
+                    if (cur < 0 && cur != kWideDone && leaf == 0) {
+                        leaf = cur;
+                        cur = stack[--sp];
+                    }
+                }
+            }
+        }
+        // the waiting triangles
+        if (leaf != 0) {
+            float t;
+            int prim;
+            const int take = wide_leaf(a, o, inv, io.direction(ray), leaf, dist, t, prim);
+            leaf = 0;
+            if (take == 1) {
+                closest = prim;
+                dist = t;
+                if (io.any(ray)) cur = kWideDone;
+            } else if (take == 2) {
+                io.mark(ray);
+                rest = true;
+                live = false;
+                cur = kWideDone;
+            }
+            if (cur < 0 && cur != kWideDone) {
+                leaf = cur;
+                cur = stack[--sp];
+            }
+        }
+        if (live && cur == kWideDone && leaf == 0) {
+            io.store(ray, closest, dist);
+            live = false;
+        }
+    }
+    // the rays set aside.  A call inside the loop made the compiler keep eight
+    // of its values in local memory (58 million reloads in a 1.1 billion
+    // instruction launch); here nothing is live across it.
+    if (!__any_sync(full, rest)) return;
+    __syncwarp();  // the marks are other lanes' stores
+    for (int at = 0;; at++) {
+        const int i = group == 32 ? at * stride + warp * 32 + lane : at == 0 && lane < group ? warp * group + lane : n;
+        if (!__any_sync(full, i < n)) break;
+        const bool want = i < n && io.marked(i);
+        if (__any_sync(full, want)) wide_rest(a, io, i, want);
+    }
 }
 
 }  // namespace zgl
