@@ -384,19 +384,22 @@ static __device__ __noinline__ void wide_rest(DeviceAccel a, Io io, int i, bool 
 //  * a lane that reaches a triangle sets it aside and goes on with the nodes
 //    behind it (a later, larger distance only adds nodes; triangles are still
 //    tested in order).  The warp turns to the waiting triangles when fewer
-//    than kInner lanes have a node left (8 to 24 measured, flat at 16 to 20).
+//    than kInner lanes have a node left, counted every second node (4M bounce
+//    rays: 12 lanes 2.83, 16 2.65, 20 2.55 ms, counting every node; every
+//    second 2.55 at 16, 2.54 at 20, 2.49 at 22 with refills from 6 idle lanes;
+//    24 lanes is faster on the large soup only).
 // 64-byte nodes in two 32-byte loads: with 128-byte nodes of full floats in
 // eight 16-byte loads the L1 was 70% busy (a gather takes a cycle a lane) and
 // the same loop ran at 760 Mrays/s.  No call in the loop: 1268 -> 1601 Mrays/s
 // (see its end).  48 registers (20 blocks of 64 threads per SM) hide more
-// latency than 56 (1485) and 40 (1447).  4M soup, 4M bounce rays: 2.62 ms,
-// 7.35 before on the threaded tables; issue slots 61% and L1 66% busy, 19 of
+// latency than 56 (1485) and 40 (1447).  4M soup, 4M bounce rays: 2.49 ms,
+// 7.35 before on the threaded tables; at 2.62 ms issue slots 61% and L1 66% busy, 19 of
 // 32 lanes active.
 constexpr int kWideBlock = 64;
 constexpr int kWideBlocksPerSM = 20;
 constexpr int64_t kWideMaxRays = int64_t(1) << 30;  // of one grid
-constexpr int kInner = 16;
-constexpr int kRefill = 8;
+constexpr int kInner = 22;
+constexpr int kRefill = 6;
 
 // Rays per warp and round: 32, fewer when n does not give 32 to eight warps
 // per SM (see wide_blocks).
@@ -489,7 +492,9 @@ __device__ __forceinline__ void wide_trace(const DeviceAccel& a, const Io& io, i
             if (__popc(inner) < kInner &&
                 (__any_sync(full, leaf != 0) || (more && __popc(__ballot_sync(full, cur == kWideDone)) >= kRefill)))
                 break;
-            if (cur >= 0) {
+#pragma unroll
+            for (int twice = 0; twice < 2; twice++) {
+                if (cur < 0) continue;
                 if (sp > kWideStack - 4) {
                     io.mark(ray);
                     rest = true;
