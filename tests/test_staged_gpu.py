@@ -97,21 +97,30 @@ def test_batch_of_staged_and_shared_requests(zgl_lib, cuda):
     batch.close()
 
 
-def test_adjoint_of_the_staged_forward(zgl_lib, cuda):
-    """The kept casts replay the staged forward's paths: the gradient is the one
-    of a replay that traces again (float atomics: 1e-5 of the largest), and the
-    image the integrator's mean."""
+@pytest.mark.parametrize("make, params", [
+    (lambda: diff_scene(seed=14, width=W, height=H), dict(max_depth=1)),
+    (lambda: diff_scene(seed=15, width=W, height=H), dict(max_depth=8, russian_roulette=1, rr_start_depth=2)),
+    (lambda: diff_scene(seed=14, width=W, height=H), dict(max_depth=11)),  # beyond the kept casts
+    (lambda: _env(diff_scene(seed=16, width=W, height=H, sampler=0)), dict(max_depth=4, light_portion=0.3,
+                                                                          light_env_uniform_sample=1)),
+    (lambda: textured_scene(seed=17, width=W, height=H, base="zoo"), dict(max_depth=6)),
+], ids=["depth_1", "depth_8", "depth_11", "environment", "textured_zoo"])
+def test_adjoint_of_the_staged_forward(zgl_lib, cuda, make, params):
+    """The replay of the kept casts, staged where they hold the whole path: the
+    gradient is the one of the one-kernel replay that traces again (float
+    atomics: 1e-5 of the largest), and the image the integrator's mean."""
     import torch
 
     n = 2
-    sc = Scene(diff_scene(seed=14, width=W, height=H))
-    r = DiffRenderer(sc, n, max_depth=11)
+    sc = Scene(make())
+    r = DiffRenderer(sc, n, **params)
     img = r.forward()
-    integ = PathIntegrator(sc, max_depth=11)
+    integ = PathIntegrator(sc, **params)
     integ.render_passes(n)
     mean = integ.get_frame()[0][..., :3] / np.float32(n)
     assert np.array_equal(img.cpu().numpy().view(np.uint32), mean.view(np.uint32))
     d_image = torch.rand((H, W, 3), device=cuda, generator=torch.Generator(cuda).manual_seed(2)) - 0.5
+    d_image[: H // 3] = 0.0  # pixels that need no replay
     kept = r.backward(d_image).cpu().numpy().astype(np.float64)
     r.set_params(r.params())  # drops the casts
     traced = r.backward(d_image).cpu().numpy().astype(np.float64)

@@ -329,6 +329,8 @@ staged_trace_kernel(const __grid_constant__ DeviceScene sc, const __grid_constan
     wide_trace(sc.accel, StagedRays{&sc, &c, &l, paths}, paths + shadows, wide_group(paths + shadows, sms));
 }
 
+}  // namespace
+
 int staged_sms() {
     static std::atomic<int> cache[64];
     int dev = 0, k = 0;
@@ -343,7 +345,11 @@ int staged_sms() {
     return k;
 }
 
-}  // namespace
+cudaError_t launch_staged_rows(const StagedPool& pool, const uint32_t* mats, int32_t row0, int32_t n,
+                               cudaStream_t st) {
+    staged_rows_kernel<<<n, 256, 0, st>>>(mats, row0, pool.rows);
+    return cudaGetLastError();
+}
 
 bool staged_alloc(StagedPool& pool, int64_t total) {
     const int64_t n = std::max<int64_t>(1, std::min(total, kStagedPaths));

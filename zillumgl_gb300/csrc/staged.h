@@ -57,6 +57,11 @@ struct StagedJob {
     uint32_t* vis;
 };
 cudaError_t launch_staged(const StagedPool& pool, const StagedJob& job, cudaStream_t st);
+// Sobol rows of samples [row0, row0 + n), n at most kStagedRows, into the pool.
+cudaError_t launch_staged_rows(const StagedPool& pool, const uint32_t* mats, int32_t row0, int32_t n,
+                               cudaStream_t st);
+// SMs of the current device.
+int staged_sms();
 
 // Whether a scene and depth run staged.
 inline bool staged_covers(const DeviceScene& sc, int32_t maxDepth) {
