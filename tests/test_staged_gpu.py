@@ -8,9 +8,11 @@ import numpy as np
 import pytest
 
 import oracle
-from zillumgl_gb300.scene import BatchRenderer, DiffRenderer, PathIntegrator, Scene
+from zillumgl_gb300.scene import BatchRenderer, DiffRenderer, LightIntegrator, PathIntegrator, Scene, TripleIntegrator
 from zillumgl_gb300.synthetic import (city_scene, cornell_scene, diff_scene, material_zoo_scene, sky_environment,
                                       sphere_box_scene, textured_scene)
+
+from tests.test_light_gpu import _check
 
 pytestmark = pytest.mark.gpu
 
@@ -128,3 +130,28 @@ def test_adjoint_of_the_staged_forward(zgl_lib, cuda, make, params):
     assert np.abs(kept - traced).max() <= 1e-5 * np.abs(traced).max()
     for x in (r, integ, sc):
         x.close()
+
+
+@pytest.mark.parametrize("make", [
+    lambda: cornell_scene(seed=31, width=96, height=80),
+    lambda: textured_scene(seed=32, width=90, height=70, base="zoo"),
+    lambda: city_scene(seed=33, width=96, height=54, grid=12, n_spheres=40, env_size=(16, 8)),
+], ids=["cornell", "textured_zoo", "city"])
+@pytest.mark.parametrize("triple", [False, True])
+@pytest.mark.parametrize("params", [dict(max_depth=1), dict(max_depth=6, russian_roulette=1, rr_start_depth=2)],
+                         ids=["depth_1", "roulette"])
+def test_light_paths_equal_the_oracle(zgl_lib, cuda, make, triple, params):
+    """98,304 light paths a pass run staged; film sums within the 1e-4 that
+    float atomics are held to."""
+    data = make()
+    sc = Scene(data)
+    params = dict(params, blocks_per_pass=64)
+    integ = (TripleIntegrator if triple else LightIntegrator)(sc, **params)
+    integ.render_passes(2)
+    got = integ.get_frame()[0][..., :3]
+    orc = oracle.OracleScene(data, sc.export("sobol"), params)
+    ref = orc.render_triple(2, blocks=64) if triple else orc.render_lt(2, blocks=64)
+    assert ref.sum() > 0
+    _check(got, ref)
+    integ.close()
+    sc.close()

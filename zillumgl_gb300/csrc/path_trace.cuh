@@ -52,6 +52,22 @@ __device__ __forceinline__ float pdfSelectEnv(const DeviceScene& sc, const PathP
     return pp.uniformSel ? (1.0f - pp.portion) : sc.envSum / (sc.lightSum + sc.envSum);
 }
 
+template <bool FULL>
+__device__ __forceinline__ void shadeSurface(const DeviceScene& sc, int id, v3 pos, v3 wo, Surface& surf,
+                                             uint32_t& matType, BSDFParam& mp) {
+    TriShade tri = loadTri(sc, id);
+    surf = surfaceInfo(tri, pos);
+    int matId = tri.matTex & 0x0000ffff;
+    matType = loadMaterialType(sc, matId);
+    if (matType != kDielectric && matType != kThinDielectric && dot(surf.ns, wo) < 0.0f) {
+        surf.ns = -surf.ns;
+        surf.ng = -surf.ng;
+    }
+    mp = loadMaterial<FULL>(sc, matType, tri.matTex, id, surf);
+}
+
+__device__ __forceinline__ float weightT1(float s0t1, float s1t1) { return 1.0f / (s0t1 + s1t1 + 1.0f); }
+
 // Ray casts of a path: closest hits in path order (`hit`) and the light
 // samples' occlusion tests (operator(), the TraceVis interface).  DirectCast
 // traverses the accelerator for both.

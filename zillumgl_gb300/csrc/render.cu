@@ -104,6 +104,23 @@ void staged_passes(zgl_integrator* it, int32_t f0, int32_t n, cudaStream_t st) {
     ZGL_CUDA(plain::launch_accumulate_passes(sc, it->curSample, n, it->d_passes, it->d_frame, st));
 }
 
+// The light paths of one pass, staged.
+void staged_light(zgl_integrator* it, uint32_t paths, bool triple, cudaStream_t st) {
+    const zgl_scene* sc = it->scene;
+    StagedLightJob job{};
+    job.sc = sc->view();
+    job.maxDepth = it->params.max_depth;
+    job.rr = it->params.russian_roulette;
+    job.rrStart = it->params.rr_start_depth;
+    job.full = sc->fullMaterials;
+    job.triple = triple;
+    job.paths = paths;
+    job.seed = (uint32_t)it->curSample * paths + (uint32_t)it->freeCounter;
+    job.scale = plain::triple_scale(sc, it->blocks, 1);
+    job.film = it->d_film;
+    ZGL_CUDA(launch_staged_light(it->pool, job, st));
+}
+
 }  // namespace
 
 extern "C" {
@@ -169,6 +186,11 @@ zgl_status zgl_integrator_create(zgl_scene* scene, int32_t kind, const zgl_integ
             e = cudaSuccess;
         }
     }
+    // light paths in one launch each (loops continue a thread's random stream)
+    const int64_t lightPaths = 1536 * (int64_t)it->blocks;
+    if (e == cudaSuccess && kind != ZGL_INTEGRATOR_PATH && it->loops == 1 && p.max_depth >= 1 &&
+        staged_covers(scene->view(), p.max_depth) && staged_light_pays(scene->view(), lightPaths))
+        staged_alloc(it->pool, lightPaths);  // without the memory: one kernel
     if (e != cudaSuccess) {
         if (it->d_frame) cudaFree(it->d_frame);
         if (it->d_film) cudaFree(it->d_film);
@@ -202,16 +224,27 @@ zgl_status zgl_integrator_render_pass(zgl_integrator* it, void* stream) {
             it->finished = true;
             return ZGL_OK;
         }
-        const auto pass = long_ray_scene(sc) ? long_rays::launch_light_pass : plain::launch_light_pass;
-        ZGL_CUDA(pass(sc, it->params, it->blocks, it->curSample, it->freeCounter, it->d_film, st));
+        if (it->pool.arena) {
+            staged_light(it, 1536u * (uint32_t)it->blocks, false, st);
+        } else {
+            const auto pass = long_ray_scene(sc) ? long_rays::launch_light_pass : plain::launch_light_pass;
+            ZGL_CUDA(pass(sc, it->params, it->blocks, it->curSample, it->freeCounter, it->d_film, st));
+        }
         it->samplePerPixel += (float)it->blocks * 1536.0f / (float)(sc->filmW * sc->filmH);
     } else {
         if (it->params.finite_sample && it->curSample > it->params.max_sample) {
             it->finished = true;
             return ZGL_OK;
         }
-        const auto pass = long_ray_scene(sc) ? long_rays::launch_triple_pass : plain::launch_triple_pass;
-        ZGL_CUDA(pass(sc, it->params, it->blocks, it->loops, it->curSample, it->freeCounter, it->d_film, st));
+        const bool large = long_ray_scene(sc);
+        const auto camera = large ? long_rays::launch_triple_camera : plain::launch_triple_camera;
+        ZGL_CUDA(camera(sc, it->params, it->curSample, it->freeCounter, it->d_film, st));
+        if (it->pool.arena) {
+            staged_light(it, 1536u * (uint32_t)it->blocks, true, st);
+        } else {
+            const auto light = large ? long_rays::launch_triple_light : plain::launch_triple_light;
+            ZGL_CUDA(light(sc, it->params, it->blocks, it->loops, it->curSample, it->freeCounter, it->d_film, st));
+        }
         it->samplePerPixel += 1.0f;
     }
     it->curSample++;

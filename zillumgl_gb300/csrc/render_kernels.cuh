@@ -211,20 +211,6 @@ __device__ __forceinline__ void accumulateFilm(const DeviceScene& sc, float* fil
     atomicAdd(p + 2, res.z);
 }
 
-template <bool FULL>
-__device__ __forceinline__ void shadeSurface(const DeviceScene& sc, int id, v3 pos, v3 wo, Surface& surf,
-                                             uint32_t& matType, BSDFParam& mp) {
-    TriShade tri = loadTri(sc, id);
-    surf = surfaceInfo(tri, pos);
-    int matId = tri.matTex & 0x0000ffff;
-    matType = loadMaterialType(sc, matId);
-    if (matType != kDielectric && matType != kThinDielectric && dot(surf.ns, wo) < 0.0f) {
-        surf.ns = -surf.ns;
-        surf.ng = -surf.ng;
-    }
-    mp = loadMaterial<FULL>(sc, matType, tri.matTex, id, surf);
-}
-
 // lightIntegTrace (light_path_integ.glsl:45-146); the light tracer forces the
 // independent sampler (LightPath.cpp:49), so every dimension is rand().
 template <bool FULL>
@@ -303,7 +289,6 @@ __device__ void lightTrace(const DeviceScene& sc, const PathParams& pp, Sampler&
 
 __device__ __forceinline__ float weightS0(float s1s0, float t1s0) { return 1.0f / (1.0f + s1s0 + t1s0); }
 __device__ __forceinline__ float weightS1(float s1s0, float t1s1) { return s1s0 / (1.0f + s1s0 + s1s0 * t1s1); }
-__device__ __forceinline__ float weightT1(float s0t1, float s1t1) { return 1.0f / (s0t1 + s1t1 + 1.0f); }
 
 // traceCameraPath (triple_path_pass_pt.glsl:59-195)
 template <bool FULL>
@@ -637,8 +622,13 @@ cudaError_t launch_light_pass(const zgl_scene* s, const zgl_integrator_params& p
     return cudaGetLastError();
 }
 
-cudaError_t launch_triple_pass(const zgl_scene* s, const zgl_integrator_params& p, int32_t blocks, int32_t loops,
-                               int32_t spp, int32_t freeCounter, float* film, cudaStream_t st) {
+// What a light path of the triple integrator weighs (uScale).
+float triple_scale(const zgl_scene* s, int32_t blocks, int32_t loops) {
+    return (float)(s->filmW * s->filmH) / (float)(blocks * loops * 1536);
+}
+
+cudaError_t launch_triple_camera(const zgl_scene* s, const zgl_integrator_params& p, int32_t spp, int32_t freeCounter,
+                                 float* film, cudaStream_t st) {
     PathParams pp{p.max_depth, p.russian_roulette, p.rr_start_depth, p.sample_light, p.light_env_uniform_sample,
                   p.light_portion};
     dim3 block(kTileX, kTileY);
@@ -647,10 +637,15 @@ cudaError_t launch_triple_pass(const zgl_scene* s, const zgl_integrator_params& 
         triple_pt_kernel<true><<<grid, block, 0, st>>>(s->view(), pp, spp, freeCounter, sample_offset(spp), film);
     else
         triple_pt_kernel<false><<<grid, block, 0, st>>>(s->view(), pp, spp, freeCounter, sample_offset(spp), film);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
+    return cudaGetLastError();
+}
+
+cudaError_t launch_triple_light(const zgl_scene* s, const zgl_integrator_params& p, int32_t blocks, int32_t loops,
+                                int32_t spp, int32_t freeCounter, float* film, cudaStream_t st) {
+    PathParams pp{p.max_depth, p.russian_roulette, p.rr_start_depth, p.sample_light, p.light_env_uniform_sample,
+                  p.light_portion};
     uint32_t n = 1536u * (uint32_t)blocks;
-    float uScale = (float)(s->filmW * s->filmH) / (float)(blocks * loops * 1536);
+    const float uScale = triple_scale(s, blocks, loops);
     if (s->fullMaterials)
         triple_lpt_kernel<true><<<(n + kLightBlock - 1) / kLightBlock, kLightBlock, 0, st>>>(
         s->view(), pp, (uint32_t)spp, (uint32_t)freeCounter, n, (uint32_t)loops, uScale, film);

@@ -23,14 +23,12 @@
 #include <atomic>
 
 #include "path_step.cuh"
-#include "staged.h"
-#include "wide.cuh"
+#include "staged.cuh"
 #include "zgl_internal.h"
 
 namespace zgl {
 namespace {
 
-constexpr unsigned kAll = 0xffffffffu;
 // Threads of a shading block: its paths are sorted by what they shade, so a
 // larger block has more uniform warps (sphere scene, 2M paths: 128 threads 714
 // us unsorted, 512 sorted 376 us, 12.6 -> 25.2 lanes and 8.2 -> 1.6
@@ -41,15 +39,6 @@ constexpr int kShadeBlock = 512;
 constexpr int kShadeBlockLarge = 1024;
 constexpr int64_t kLargePaths = 512 * 1024;
 constexpr int kStartBlock = 256;
-constexpr int kCountStride = 2;
-
-// What a launch needs of the pool: the list it reads and the one it writes.
-struct StagedLists {
-    float4 *org, *dir, *thr, *pos;
-    uint2* rng;
-    int2* hit;
-    float4 *sorg, *sdir, *scon;
-};
 
 // Items of a chunk: paths [q0, q0 + count) of the job, counted over samples
 // and 8x4 pixel tiles (a warp's camera rays are neighbours); items outside the
@@ -67,30 +56,6 @@ struct StagedChunk {
     uint32_t* vis;
     const uint32_t* rows;
 };
-
-// Position of this thread's entry in a list that `want` threads of the block
-// append to; one atomic per block.  Every thread of the block calls.
-template <int BLOCK>
-__device__ __forceinline__ uint32_t block_append(bool want, uint32_t* counter, uint32_t* sh) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const unsigned m = __ballot_sync(kAll, want);
-    if (lane == 0) sh[w] = (uint32_t)__popc(m);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t total = 0;
-#pragma unroll
-        for (int i = 0; i < BLOCK / 32; i++) {
-            const uint32_t c = sh[i];
-            sh[i] = total;
-            total += c;
-        }
-        const uint32_t base = total ? atomicAdd(counter, total) : 0u;
-#pragma unroll
-        for (int i = 0; i < BLOCK / 32; i++) sh[i] += base;
-    }
-    __syncthreads();
-    return sh[w] + (uint32_t)__popc(m & ((1u << lane) - 1u));
-}
 
 __device__ __forceinline__ void store_path(const StagedLists& l, uint32_t i, const PathState& st, const Sampler& g,
                                            uint32_t path, uint32_t casts) {
@@ -154,60 +119,6 @@ __device__ __forceinline__ int64_t path_index(const DeviceScene& sc, const Stage
     const int64_t tile = in >> 5;
     const int px = (int)(tile % c.tilesX) * 8 + ((int)in & 7), py = (int)(tile / c.tilesX) * 4 + (((int)in >> 3) & 3);
     return (int64_t)s * c.npix + (int64_t)py * sc.filmW + px;
-}
-
-// What a path's shading runs: nothing but emission (0), the vertex's material
-// type + 1, or no path (7).
-template <bool FULL>
-__device__ __forceinline__ int shade_class(const DeviceScene& sc, int id) {
-    if (id < 0 || id >= sc.objPrimCount) return 0;
-    const int matTex = __float_as_int(__ldg(reinterpret_cast<const float*>(sc.shade + 5 * (size_t)id + 4) + 2));
-    const uint32_t type = loadMaterialType(sc, matTex & 0x0000ffff);
-    return 1 + (int)min(type, FULL ? 5u : 1u);
-}
-
-// The block's paths in order of class, so that a warp's lanes shade alike:
-// thread t takes path perm[t] of the block's window.  A counting sort with one
-// ballot per class; every thread of the block calls.
-template <int BLOCK>
-struct ShadeSort {
-    uint16_t perm[BLOCK];
-    uint32_t count[8][BLOCK / 32];
-};
-template <int BLOCK>
-__device__ __forceinline__ int block_sort(int cls, ShadeSort<BLOCK>& sh) {
-    constexpr int kWarps = BLOCK / 32;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    unsigned mine = 0u;
-#pragma unroll
-    for (int c = 0; c < 8; c++) {
-        const unsigned m = __ballot_sync(kAll, cls == c);
-        if (cls == c) mine = m;
-        if (lane == c) sh.count[c][w] = (uint32_t)__popc(m);
-    }
-    __syncthreads();
-    if (w == 0) {  // exclusive sums, class-major
-        uint32_t v[(8 * kWarps + 31) / 32], total = 0;
-        constexpr int kPer = (8 * kWarps + 31) / 32;
-        uint32_t* flat = &sh.count[0][0];
-#pragma unroll
-        for (int k = 0; k < kPer; k++) {
-            v[k] = total;
-            total += flat[lane * kPer + k];
-        }
-        uint32_t x = total;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t y = __shfl_up_sync(kAll, x, d);
-            if (lane >= d) x += y;
-        }
-#pragma unroll
-        for (int k = 0; k < kPer; k++) flat[lane * kPer + k] = x - total + v[k];
-    }
-    __syncthreads();
-    sh.perm[sh.count[cls][w] + (uint32_t)__popc(mine & ((1u << lane) - 1u))] = (uint16_t)threadIdx.x;
-    __syncthreads();
-    return sh.perm[threadIdx.x];
 }
 
 // One step of every path of the list: step 0 takes the camera rays' hits.
@@ -278,7 +189,6 @@ staged_shade_kernel(const __grid_constant__ DeviceScene sc, const __grid_constan
 }
 
 // The rays of one step: the live paths' first, then the shadow rays.
-constexpr uint32_t kSetAside = 0x80000000u;
 struct StagedRays {
     static constexpr bool kClosest = true, kAny = true;
     const DeviceScene* sc;
@@ -405,10 +315,7 @@ cudaError_t launch_staged(const StagedPool& pool, const StagedJob& job, cudaStre
     c.castDepth = job.castDepth;
     c.vis = job.vis;
     c.rows = pool.rows;
-    StagedLists lists[2];
-    for (int i = 0; i < 2; i++)
-        lists[i] = StagedLists{pool.org[i], pool.dir[i], pool.thr[i], pool.pos[i], pool.rng[i],
-                               pool.hit,    pool.sorg,   pool.sdir,   pool.scon};
+    const StagedLists lists[2] = {staged_list(pool, 0), staged_list(pool, 1)};
     const int64_t total = c.perSample * job.n;
     for (c.q0 = 0; c.q0 < total; c.q0 += c.count) {
         c.count = std::min(total - c.q0, pool.paths);

@@ -358,64 +358,82 @@ __device__ __forceinline__ bool traverse_lane_m(const DeviceAccel& a, const Trac
 }
 
 // The rest of one ray from entry k, walked by all 32 lanes of the warp (ray
-// and state warp-uniform; every lane calls).
+// and state warp-uniform; every lane calls).  Four windows of 32 entries are
+// loaded and tested at once, so that the walk waits for memory once per 128
+// entries: a dense walk is nothing but that latency (1.6 us a window of 32).
 template <bool ANY, int MODE>
 __device__ __forceinline__ void traverse_warp(const DeviceAccel& a, const TraceRay& r, float& dist, int& k,
                                               int& closest) {
+    constexpr int kWindows = 4;
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const float4* __restrict__ base = a.nodes + (size_t)r.face * (size_t)a.M * 2;
     const int M = a.M;
     while (k < M) {
-        const int j = k + lane;
-        float4 lo = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(-1)), hi = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (j < M) {
-            lo = __ldg(base + 2 * (size_t)j);
-            hi = __ldg(base + 2 * (size_t)j + 1);
+        const int first = k;
+        float4 lo[kWindows], hi[kWindows];
+#pragma unroll
+        for (int w = 0; w < kWindows; w++) {
+            const int j = min(first + 32 * w + lane, M - 1);
+            lo[w] = __ldg(base + 2 * (size_t)j);
+            hi[w] = __ldg(base + 2 * (size_t)j + 1);
         }
-        float tmin = 0.0f, t = 0.0f;
-        const bool geom = j < M && box_hit_m<MODE>(lo, hi, r, tmin);
-        const int prim = __float_as_int(lo.w);
-        const bool tri = geom && prim >= 0 && tri_hit(a.tris, prim, r, t);
-        const int skip = max(__float_as_int(hi.w), j + 1);
-        unsigned H = __ballot_sync(full, geom && !(tmin > dist)), T = __ballot_sync(full, tri);
-        // The path through the window, from miss to miss: the hits up to the
-        // next miss are consecutive entries, and only a triangle among them
-        // can change the distance.  p only grows.
-        int p = 0;
-        for (;;) {
-            const unsigned from = 0xffffffffu << p;
-            const unsigned miss = ~H & from;
-            const int q = miss ? __ffs(miss) - 1 : 32;
-            const unsigned cand = T & H & from & (q < 32 ? (1u << q) - 1u : 0xffffffffu);
-            if (cand) {
-                const int c = __ffs(cand) - 1;
-                const float tt = __shfl_sync(full, t, c);
-                if (tt < dist) {
-                    closest = __shfl_sync(full, prim, c);
-                    if (ANY) {
-                        k = M;
-                        return;
+        float tmin[kWindows], t[kWindows];
+        int prim[kWindows], skip[kWindows];
+        bool geom[kWindows], tri[kWindows];
+#pragma unroll
+        for (int w = 0; w < kWindows; w++) {
+            const int j = first + 32 * w + lane;
+            tmin[w] = t[w] = 0.0f;
+            geom[w] = j < M && box_hit_m<MODE>(lo[w], hi[w], r, tmin[w]);
+            prim[w] = __float_as_int(lo[w].w);
+            skip[w] = max(__float_as_int(hi[w].w), j + 1);
+        }
+#pragma unroll
+        for (int w = 0; w < kWindows; w++) tri[w] = geom[w] && prim[w] >= 0 && tri_hit(a.tris, prim[w], r, t[w]);
+#pragma unroll
+        for (int w = 0; w < kWindows; w++) {
+            const int start = first + 32 * w;  // k is here or beyond
+            if (k >= start + 32 || k >= M) continue;
+            unsigned H = __ballot_sync(full, geom[w] && !(tmin[w] > dist)), T = __ballot_sync(full, tri[w]);
+            // The path through the window, from miss to miss: the hits up to
+            // the next miss are consecutive entries, and only a triangle among
+            // them can change the distance.  p only grows.
+            int p = k - start;
+            for (;;) {
+                const unsigned from = 0xffffffffu << p;
+                const unsigned miss = ~H & from;
+                const int q = miss ? __ffs(miss) - 1 : 32;
+                const unsigned cand = T & H & from & (q < 32 ? (1u << q) - 1u : 0xffffffffu);
+                if (cand) {
+                    const int c = __ffs(cand) - 1;
+                    const float tt = __shfl_sync(full, t[w], c);
+                    if (tt < dist) {
+                        closest = __shfl_sync(full, prim[w], c);
+                        if (ANY) {
+                            k = M;
+                            return;
+                        }
+                        dist = tt;
+                        H = __ballot_sync(full, geom[w] && !(tmin[w] > dist));
                     }
-                    dist = tt;
-                    H = __ballot_sync(full, geom && !(tmin > dist));
+                    T &= ~(1u << c);
+                    p = c + 1;
+                    if (p < 32) continue;
+                    k = start + 32;
+                    break;
                 }
-                T &= ~(1u << c);
-                p = c + 1;
-                if (p < 32) continue;
-                k += 32;
-                break;
+                if (q == 32) {
+                    k = start + 32;
+                    break;
+                }
+                const int next = __shfl_sync(full, skip[w], q);
+                if (next >= M || next - start >= 32) {
+                    k = next;
+                    break;
+                }
+                p = next - start;
             }
-            if (q == 32) {
-                k += 32;
-                break;
-            }
-            const int next = __shfl_sync(full, skip, q);
-            if (next >= M || next - k >= 32) {
-                k = next;
-                break;
-            }
-            p = next - k;
         }
     }
 }
