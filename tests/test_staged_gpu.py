@@ -155,3 +155,34 @@ def test_light_paths_equal_the_oracle(zgl_lib, cuda, make, triple, params):
     _check(got, ref)
     integ.close()
     sc.close()
+
+
+# Calls near the smallest that run staged, and on both sides of the small shading blocks' line (77,824 paths).
+SMALL = {
+    "spheres_one_pass": (lambda: sphere_box_scene(31, 30000, 47, 45), dict(max_depth=5), 1),
+    "cornell_three_passes": (lambda: cornell_scene(seed=32, width=57, height=49), dict(max_depth=5), 3),
+    "cornell_below": (lambda: cornell_scene(seed=33, width=277, height=278), dict(max_depth=3), 1),
+    "cornell_above": (lambda: cornell_scene(seed=33, width=279, height=281), dict(max_depth=3), 1),
+    "zoo_one_pass": (lambda: material_zoo_scene(seed=34, width=191, height=173), dict(max_depth=4), 1),
+    "textured_two_passes": (lambda: textured_scene(seed=35, width=67, height=63, base="zoo"), dict(max_depth=4), 2),
+}
+
+
+@pytest.mark.parametrize("name", list(SMALL))
+def test_small_calls_equal_the_oracle(zgl_lib, cuda, name):
+    make, params, n = SMALL[name]
+    data = make()
+    sc = Scene(data)
+    w, h = data.film
+    orc = oracle.OracleScene(data, sc.export("sobol"), params)
+    pix = np.random.default_rng(2).choice(w * h, 1500, replace=False).astype(np.int32)
+    ref = orc.render_pt(pix, n)
+    it = PathIntegrator(sc, **params)
+    if n == 1:
+        it.render_one_pass()
+    else:
+        it.render_passes(n)
+    got = it.get_frame()[0][..., :3].reshape(-1, 3)[pix]
+    assert np.array_equal(got.view(np.uint32), ref.view(np.uint32))
+    for x in (it, sc):
+        x.close()

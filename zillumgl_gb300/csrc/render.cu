@@ -79,7 +79,8 @@ bool is_device_memory(const void* p) {
 bool runs_staged(const zgl_integrator* it, int64_t n) {
     const zgl_scene* sc = it->scene;
     const int64_t paths = (int64_t)sc->filmW * sc->filmH * n;
-    return it->pool.arena != nullptr && !long_ray_scene(sc) && it->passesCap >= (size_t)(3 * paths) && staged_pays(sc->view(), paths);
+    return it->pool.arena != nullptr && !long_ray_scene(sc) && it->passesCap >= (size_t)(3 * paths) &&
+           staged_pays(sc->view(), paths, n > 1, sc->fullMaterials);
 }
 
 // Passes [curSample, curSample + n) of the path tracer, staged.  `f0` is the
@@ -173,7 +174,7 @@ zgl_status zgl_integrator_create(zgl_scene* scene, int32_t kind, const zgl_integ
     }
     if (e == cudaSuccess && kind == ZGL_INTEGRATOR_PATH && !long_ray_scene(scene) &&
         staged_covers(scene->view(), p.max_depth) &&
-        staged_pays(scene->view(), (int64_t)npix)) {
+        staged_pays(scene->view(), (int64_t)npix, false, scene->fullMaterials)) {
         // room for one pass now, so that a pass allocates nothing; without it
         // the one-kernel path tracer runs
         it->passesCap = 3 * npix;
@@ -281,7 +282,7 @@ zgl_status zgl_integrator_render_passes(zgl_integrator* it, int32_t passes, void
         }
         const int64_t paths = std::min(staged_paths(sc->filmW, sc->filmH, n), kStagedPaths);
         if (!long_ray_scene(sc) && staged_covers(sc->view(), it->params.max_depth) &&
-            staged_pays(sc->view(), (int64_t)sc->filmW * sc->filmH * n) && it->pool.paths < paths)
+            staged_pays(sc->view(), (int64_t)sc->filmW * sc->filmH * n, n > 1, sc->fullMaterials) && it->pool.paths < paths)
             staged_alloc(it->pool, paths);  // without the memory: the smaller pool, or one kernel
         if (runs_staged(it, n)) {
             staged_passes(it, f0, n, (cudaStream_t)stream);

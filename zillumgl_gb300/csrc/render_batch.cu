@@ -490,7 +490,7 @@ void check_config(const zgl_batch_config& c) {
 
 // Whether n samples of a request run on the staged path tracer.
 bool runs_staged(const BatchRequest& q, int n) {
-    return staged_covers(q.sc, q.pp.maxDepth) && staged_pays(q.sc, (int64_t)q.npix * n);
+    return staged_covers(q.sc, q.pp.maxDepth) && staged_pays_in_batch(q.sc, (int64_t)q.npix * n);
 }
 
 // Enqueues the whole render on `st`: frame clears, then per chunk of sample

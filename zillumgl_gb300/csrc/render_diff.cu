@@ -839,7 +839,7 @@ zgl_status zgl_diff_create(zgl_scene* scene, const zgl_integrator_params* params
             ZGL_CUDA(cudaMalloc(&d->d_hits, sizeof(int2) * kCastDepth * paths));
             ZGL_CUDA(cudaMalloc(&d->d_vis, sizeof(uint32_t) * paths));
         }
-        if (staged_covers(scene->view(), d->params.max_depth) && staged_pays(scene->view(), (int64_t)paths))
+        if (staged_covers(scene->view(), d->params.max_depth) && staged_diff_pays((int64_t)paths))
             staged_alloc(d->pool, staged_paths(scene->filmW, scene->filmH, spp));
         std::vector<int32_t> inst((size_t)std::max(scene->nLight, 1), 0);
         for (int k = 0; k < d->ninst; k++)

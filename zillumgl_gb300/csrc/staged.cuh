@@ -64,6 +64,7 @@ __device__ __forceinline__ int shade_class(const DeviceScene& sc, int id) {
 // ballot per class; every thread of the block calls.
 template <int BLOCK>
 struct ShadeSort {
+    static_assert(BLOCK >= 128, "the scan reads a whole warp's number of counters");
     uint16_t perm[BLOCK];
     uint32_t count[8][BLOCK / 32];
 };

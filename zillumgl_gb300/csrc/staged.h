@@ -81,11 +81,26 @@ int staged_sms();
 inline bool staged_covers(const DeviceScene& sc, int32_t maxDepth) {
     return sc.accel.wide != nullptr && maxDepth >= 0 && maxDepth <= kStagedMaxDepth;
 }
-// Whether it is the faster way for a call of `paths` paths.  Two launches a
-// bounce have a latency that few paths do not fill: on a 2k-triangle box 65k
-// paths take 0.47 ms staged and 0.40 in one kernel, 147k 0.59 and 0.73; on
-// 100k triangles 16k paths take 0.59 and 0.69, 65k 0.68 and 0.75.
-inline bool staged_pays(const DeviceScene& sc, int64_t paths) {
+// Whether it is the faster way for a call of `paths` paths, in one pass or
+// several.  Two launches a bounce have a latency (about 65 us at depth 5) that
+// few paths do not fill.  One kernel and staged, us, one pass: 2k triangles,
+// Lambertian and principled, 32k paths 314 and 384, 65k 400 and 406, 90k 505
+// and 452; all material types 16k 328 and 390, 32k 446 and 428; 100k triangles
+// 2k 525 and 380, 65k 755 and 606; 60k triangles 2k 642 and 431, 32k 675 and
+// 677.  The kernel of several passes has 32 registers: 9k paths on 2k
+// triangles 342 and 317, on all material types 383 and 357.
+inline bool staged_pays(const DeviceScene& sc, int64_t paths, bool several, bool full) {
+    if (several) return paths >= 8192;
+    if (sc.accel.M >= 16384) return paths >= 2048;
+    return paths >= (full ? 32768 : 73728);
+}
+// A differentiable step, forward and replay (2k triangles, depth 6, us): 16k
+// paths 702 in one kernel each and 709 staged, 33k 789 and 767, 65k 1043 and
+// 842.
+inline bool staged_diff_pays(int64_t paths) { return paths >= 32768; }
+// Whether a request of a batch leaves the launch it shares with the others:
+// what fills the GPU there is the others' paths too.
+inline bool staged_pays_in_batch(const DeviceScene& sc, int64_t paths) {
     return paths >= 98304 || (sc.accel.M >= 16384 && paths >= 32768);
 }
 // The same for light paths (depth 8; one kernel, staged): 49k on 20k triangles

@@ -387,7 +387,9 @@ static __device__ __noinline__ void wide_rest(DeviceAccel a, Io io, int i, bool 
 //    than kInner lanes have a node left, counted every second node (4M bounce
 //    rays: 12 lanes 2.83, 16 2.65, 20 2.55 ms, counting every node; every
 //    second 2.55 at 16, 2.54 at 20, 2.49 at 22 with refills from 6 idle lanes;
-//    24 lanes is faster on the large soup only).
+//    24 lanes is faster on the large soup only).  With fewer rays the number
+//    goes down with them: 65k rays on 4096 triangles 97 -> 93 us, six launches
+//    of a Cornell view's bounces 44 -> 41 us each.
 // 64-byte nodes in two 32-byte loads: with 128-byte nodes of full floats in
 // eight 16-byte loads the L1 was 70% busy (a gather takes a cycle a lane) and
 // the same loop ran at 760 Mrays/s.  No call in the loop: 1268 -> 1601 Mrays/s
@@ -484,12 +486,14 @@ __device__ __forceinline__ void wide_trace(const DeviceAccel& a, const Io& io, i
                 }
             }
         }
+        // of the lanes with a ray: few have any in a small launch, and at the end
+        const int few = min(kInner, 27 * __popc(__ballot_sync(full, live)) >> 5);
         // nodes, until few lanes have one and some wait with a triangle or
         // could be refilled
         for (;;) {
             const unsigned inner = __ballot_sync(full, cur >= 0);
             if (inner == 0u) break;
-            if (__popc(inner) < kInner &&
+            if (__popc(inner) < few &&
                 (__any_sync(full, leaf != 0) || (more && __popc(__ballot_sync(full, cur == kWideDone)) >= kRefill)))
                 break;
 #pragma unroll
