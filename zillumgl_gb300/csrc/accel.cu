@@ -504,8 +504,8 @@ private:
     int prev_ = 0, dev_ = 0;
 };
 
-// The schedule a trace call runs (ZGL_TRACE_AUTO: one thread per ray, long
-// rays finished by their warps).
+// The schedule a trace call runs (ZGL_TRACE_AUTO: the wide tree, where there
+// is one).
 int trace_schedule(const zgl_accel* a) { return a->trace_schedule; }
 
 int host_threads() {
@@ -614,7 +614,6 @@ zgl_accel* accel_create_device(const float* vertices, int64_t nv, const uint32_t
                 arena.take(a->d_nodes, 12 * a->M);
                 arena.take(a->d_tris, 3 * ntri);
                 arena.take(a->d_dfs, 2 * a->M);
-                arena.take(a->d_hit, 18 * a->M);
                 if (ntri > 1) {
                     arena.take(a->d_wide, 4 * (ntri - 1));
                     arena.take(a->d_wtris, 4 * ntri);
@@ -646,7 +645,6 @@ void accel_free(zgl_accel* a) {
         cudaFree(a->d_arena);
     } else {
         if (a->d_dfs) cudaFree(a->d_dfs);
-        if (a->d_hit) cudaFree(a->d_hit);
         if (a->d_wide) cudaFree(a->d_wide);
         if (a->d_wtris) cudaFree(a->d_wtris);
         if (a->d_counter) cudaFree(a->d_counter);
@@ -739,8 +737,7 @@ zgl_status zgl_accel_export(const zgl_accel* accel, float* bounds, int32_t* hit_
     if (accel->M > 0 && (!bounds || !hit_table))
         fail(ZGL_ERR_INVALID_ARG, "zgl_accel_export: NULL output array");
     if (accel->M > 0 && accel->device_built) {
-        export_bounds(accel->d_dfs, accel->M, bounds);
-        ZGL_CUDA(cudaMemcpy(hit_table, accel->d_hit, sizeof(int32_t) * accel->M * 18, cudaMemcpyDeviceToHost));
+        export_device_tree(accel, bounds, hit_table);
     } else if (accel->M > 0) {
         std::memcpy(bounds, accel->host.bounds.data(), sizeof(float) * accel->M * 6);
         std::memcpy(hit_table, accel->host.hitTable.data(), sizeof(int32_t) * accel->M * 18);

@@ -89,7 +89,6 @@ struct Out {
     float4* nodes;     // [6][M][2]
     float4* dfs;       // [M][2]
     float* l2;         // [M]
-    int32_t* hit;      // [6][M][3]
     int64_t M;
 };
 
@@ -156,17 +155,15 @@ __device__ __forceinline__ float diag2(const float lo[3], const float hi[3]) {
 
 // Writes node `offset` (bounds lo/hi, prim or -1, subtree size) into face
 // f's table at index pos; lanes f = 0..5 of the caller each write one face.
+// In the table an inner node's prim is ~offset.
 // Face 0's lane also writes the DFS record: `leaves` leaves come before the
 // node, `odd` is its depth's parity.
 __device__ __forceinline__ void write_entry(const Out& o, int f, int32_t pos, int32_t offset, int32_t prim,
                                             int32_t size, int32_t leaves, int odd, const float lo[3],
                                             const float hi[3]) {
     int64_t e = (int64_t)f * o.M + pos;
-    o.nodes[2 * e + 0] = make_float4(lo[0], lo[1], lo[2], __int_as_float(prim));
+    o.nodes[2 * e + 0] = make_float4(lo[0], lo[1], lo[2], __int_as_float(prim < 0 ? ~offset : prim));
     o.nodes[2 * e + 1] = make_float4(hi[0], hi[1], hi[2], __int_as_float(pos + size));
-    o.hit[3 * e + 0] = offset;
-    o.hit[3 * e + 1] = prim;
-    o.hit[3 * e + 2] = pos + size;
     if (f == 0) {
         const uint32_t w0 = prim < 0 ? (uint32_t)size : ((uint32_t)prim | 0x80000000u);
         const uint32_t w1 = (uint32_t)leaves | ((uint32_t)odd << 31);
@@ -950,15 +947,15 @@ int gpu_build_default_small() { return kDefaultSmall; }
 int gpu_build_max_small() { return kMaxSmall; }
 
 // Builds the MTBVH of the accelerator's triangles on the current device
-// (vertices and indices are device-accessible): d_nodes, d_tris, d_dfs, d_hit
-// and the wide tree.  Synchronous on `s`; throws zgl::Error.
+// (vertices and indices are device-accessible): d_nodes, d_tris, d_dfs and
+// the wide tree.  Synchronous on `s`; throws zgl::Error.
 void build_bvh_device(const float* v, int64_t nv, const uint32_t* idx, int small, zgl_accel* a, cudaStream_t s) {
     const int64_t ntri = a->ntri;
     if (ntri <= 0) return;
     if (small <= 0) small = kDefaultSmall;
     small = std::max(8, std::min(small, kMaxSmall));
     Scratch w(ntri, small);
-    Out o{a->d_nodes, a->d_dfs, w.l2, a->d_hit, a->M};
+    Out o{a->d_nodes, a->d_dfs, w.l2, a->M};
     float4* const tris = a->d_tris;
 
     int dev = 0, sms = 1;
