@@ -39,8 +39,8 @@ constexpr int kShadeBlock = 512;
 constexpr int kShadeBlockLarge = 1024;
 constexpr int64_t kLargePaths = 512 * 1024;
 // Fewer paths than four blocks of 128 per SM are shaded by such blocks, on
-// every SM and with 128 registers: 30 -> 22 us a launch at 65k paths (a
-// Cornell view 424 -> 406 us), 9k paths 340 -> 315 us.  64 registers in blocks
+// every SM and with 128 registers: a Cornell pass of 65k paths 424 -> 406 us,
+// of 9k paths 340 -> 315 us.  64 registers in blocks
 // of 256: 409.
 constexpr int kShadeBlockSmall = 128;
 constexpr int kShadeSmallPerSM = 4;

@@ -388,8 +388,8 @@ static __device__ __noinline__ void wide_rest(DeviceAccel a, Io io, int i, bool 
 //    rays: 12 lanes 2.83, 16 2.65, 20 2.55 ms, counting every node; every
 //    second 2.55 at 16, 2.54 at 20, 2.49 at 22 with refills from 6 idle lanes;
 //    24 lanes is faster on the large soup only).  With fewer rays the number
-//    goes down with them: 65k rays on 4096 triangles 97 -> 93 us, six launches
-//    of a Cornell view's bounces 44 -> 41 us each.
+//    goes down with them: 65k rays on 4096 triangles 98 -> 93 us, a
+//    256x256 Cornell pass (six launches) 453 -> 424 us.
 // 64-byte nodes in two 32-byte loads: with 128-byte nodes of full floats in
 // eight 16-byte loads the L1 was 70% busy (a gather takes a cycle a lane) and
 // the same loop ran at 760 Mrays/s.  No call in the loop: 1268 -> 1601 Mrays/s
