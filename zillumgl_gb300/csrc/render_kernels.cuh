@@ -33,15 +33,23 @@ namespace ZGL_RENDER_NS {
 namespace {
 
 // main() of path_integ_naive.glsl:145-174; MINB = minimum resident blocks
-// per SM (1: uncapped registers, kOccupied: full occupancy)
-template <bool FULL, int MINB>
+// per SM (1: uncapped registers, kOccupied: full occupancy).  THIN: only
+// `lanes` (4, 8 or 16) lanes of a warp have a path, two rows of lanes / 2
+// pixels, the block's four warps two by two.
+template <bool FULL, int MINB, bool THIN = false>
 __global__ void __launch_bounds__(kTileX* kTileY, MINB)
 path_kernel(DeviceScene sc, PathParams pp, int32_t spp, int32_t freeCounter, uint32_t sampleOffset,
-            float4* __restrict__ frame) {
+            float4* __restrict__ frame, int lanes) {
     __shared__ uint32_t row[256];
     load_sobol_row(sc, sampleOffset, row);
-    const int px = blockIdx.x * kTileX + threadIdx.x;
-    const int py = blockIdx.y * kTileY + threadIdx.y;
+    int px = blockIdx.x * kTileX + threadIdx.x;
+    int py = blockIdx.y * kTileY + threadIdx.y;
+    if (THIN) {
+        const int t = threadIdx.y * kTileX + threadIdx.x, w = t >> 5, l = t & 31, cols = lanes >> 1;
+        if (l >= lanes) return;
+        px = ((int)blockIdx.x * 2 + (w & 1)) * cols + l % cols;
+        py = ((int)blockIdx.y * 2 + (w >> 1)) * 2 + l / cols;
+    }
     if (px >= sc.filmW || py >= sc.filmH) return;
     const size_t pix = (size_t)py * sc.filmW + px;
     const uint2 seed = __ldg(&sc.pixelSeeds[pix]);
@@ -83,6 +91,20 @@ int sm_count() {
         if (cached) cache[dev].store(n, std::memory_order_relaxed);
     }
     return n;
+}
+
+// Paths of a warp for a pass of few paths: the warp runs every branch that one
+// of its paths takes, so where warps are few anyway they are filled thinner, as
+// long as that gives at most 8 warps per SM (4 with the code of every material
+// type).  One pass at depth 5, us, with 32, 16, 8, 4 paths a warp: box 32x32
+// 272 228 198 173, 64x64 270 238 212 205, 90x90 292 251 231 246, 128x128 280
+// 274 289 364, 150x150 293 306 341 466; every material 64x64 312 273 239 255,
+// 90x90 319 288 313 330, 128x128 328 358 424 562.
+int path_lanes(int64_t paths, bool full) {
+    const int64_t warps = (int64_t)sm_count() * (full ? 4 : 8);
+    for (int lanes = 4; lanes < 32; lanes *= 2)
+        if ((paths + lanes - 1) / lanes <= warps) return lanes;
+    return 32;
 }
 
 // Occupancy: the integrator kernels are bound by instruction fetch and
@@ -565,12 +587,16 @@ cudaError_t launch_path_pass(const zgl_scene* s, const zgl_integrator_params& p,
     const bool fills = (int64_t)grid.x * grid.y >= 8 * (int64_t)sm_count();
     const DeviceScene v = s->view();
     const uint32_t off = sample_offset(spp);
+    const int lanes = ZGL_LONG_RAYS ? 32 : path_lanes((int64_t)s->filmW * s->filmH, s->fullMaterials);
+    const dim3 thin((unsigned)((s->filmW + lanes - 1) / lanes), (unsigned)((s->filmH + 3) / 4));
     if (s->fullMaterials) {
-        if (fills) path_kernel<true, kOccupied><<<grid, block, 0, st>>>(v, pp, spp, freeCounter, off, frame);
-        else path_kernel<true, 1><<<grid, block, 0, st>>>(v, pp, spp, freeCounter, off, frame);
+        if (lanes < 32) path_kernel<true, 1, true><<<thin, block, 0, st>>>(v, pp, spp, freeCounter, off, frame, lanes);
+        else if (fills) path_kernel<true, kOccupied><<<grid, block, 0, st>>>(v, pp, spp, freeCounter, off, frame, 32);
+        else path_kernel<true, 1><<<grid, block, 0, st>>>(v, pp, spp, freeCounter, off, frame, 32);
     } else {
-        if (fills) path_kernel<false, kOccupied><<<grid, block, 0, st>>>(v, pp, spp, freeCounter, off, frame);
-        else path_kernel<false, 1><<<grid, block, 0, st>>>(v, pp, spp, freeCounter, off, frame);
+        if (lanes < 32) path_kernel<false, 1, true><<<thin, block, 0, st>>>(v, pp, spp, freeCounter, off, frame, lanes);
+        else if (fills) path_kernel<false, kOccupied><<<grid, block, 0, st>>>(v, pp, spp, freeCounter, off, frame, 32);
+        else path_kernel<false, 1><<<grid, block, 0, st>>>(v, pp, spp, freeCounter, off, frame, 32);
     }
     return cudaGetLastError();
 }

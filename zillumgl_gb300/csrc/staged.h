@@ -86,12 +86,12 @@ inline bool staged_covers(const DeviceScene& sc, int32_t maxDepth) {
 // few paths do not fill.  One kernel and staged, us, one pass: 2k triangles,
 // Lambertian and principled, 32k paths 314 and 384, 65k 400 and 406, 90k 505
 // and 452; all material types 16k 328 and 390, 32k 446 and 428; 100k triangles
-// 2k 525 and 380, 65k 755 and 606; 60k triangles 2k 642 and 431, 32k 675 and
-// 677.  The kernel of several passes has 32 registers: 9k paths on 2k
+// 4k 350 and 406, 16k 456 and 507, 32k 650 and 558; 60k triangles 4k 357 and
+// 458, 16k 548 and 615, 32k 675 and 675, 65k 875 and 764.  The kernel of several passes has 32 registers: 9k paths on 2k
 // triangles 342 and 317, on all material types 383 and 357.
 inline bool staged_pays(const DeviceScene& sc, int64_t paths, bool several, bool full) {
     if (several) return paths >= 8192;
-    if (sc.accel.M >= 16384) return paths >= 2048;
+    if (sc.accel.M >= 16384) return paths >= 24576;
     return paths >= (full ? 32768 : 73728);
 }
 // A differentiable step, forward and replay (2k triangles, depth 6, us): 16k
