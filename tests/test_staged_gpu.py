@@ -161,9 +161,9 @@ def test_light_paths_equal_the_oracle(zgl_lib, cuda, make, triple, params):
 SMALL = {
     "spheres_one_pass": (lambda: sphere_box_scene(31, 30000, 47, 45), dict(max_depth=5), 1),
     "cornell_three_passes": (lambda: cornell_scene(seed=32, width=57, height=49), dict(max_depth=5), 3),
-    "cornell_below": (lambda: cornell_scene(seed=33, width=277, height=278), dict(max_depth=3), 1),
-    "cornell_above": (lambda: cornell_scene(seed=33, width=279, height=281), dict(max_depth=3), 1),
-    "zoo_one_pass": (lambda: material_zoo_scene(seed=34, width=191, height=173), dict(max_depth=4), 1),
+    "cornell_below": (lambda: cornell_scene(seed=33, width=192, height=200), dict(max_depth=3), 2),
+    "cornell_above": (lambda: cornell_scene(seed=33, width=197, height=199), dict(max_depth=3), 2),
+    "zoo_one_pass": (lambda: material_zoo_scene(seed=34, width=391, height=373), dict(max_depth=4), 1),
     "textured_two_passes": (lambda: textured_scene(seed=35, width=67, height=63, base="zoo"), dict(max_depth=4), 2),
 }
 
@@ -175,7 +175,7 @@ SMALL.update({
                     (cornell_scene, 131, 123), (cornell_scene, 133, 131), (material_zoo_scene, 49, 47),
                     (material_zoo_scene, 71, 67), (material_zoo_scene, 99, 98))
 })
-SMALL["spheres_staged"] = (lambda: sphere_box_scene(37, 30000, 161, 157), dict(max_depth=5), 1)
+SMALL["spheres_staged"] = (lambda: sphere_box_scene(37, 30000, 191, 181), dict(max_depth=5), 1)
 
 
 @pytest.mark.parametrize("name", list(SMALL))

@@ -83,16 +83,19 @@ inline bool staged_covers(const DeviceScene& sc, int32_t maxDepth) {
 }
 // Whether it is the faster way for a call of `paths` paths, in one pass or
 // several.  Two launches a bounce have a latency (about 65 us at depth 5) that
-// few paths do not fill.  One kernel and staged, us, one pass: 2k triangles,
-// Lambertian and principled, 32k paths 314 and 384, 65k 400 and 406, 90k 505
-// and 452; all material types 16k 328 and 390, 32k 446 and 428; 100k triangles
-// 4k 350 and 406, 16k 456 and 507, 32k 650 and 558; 60k triangles 4k 357 and
-// 458, 16k 548 and 615, 32k 675 and 675, 65k 875 and 764.  The kernel of several passes has 32 registers: 9k paths on 2k
-// triangles 342 and 317, on all material types 383 and 357.
+// few paths do not fill, all the less where many of them miss the scene.  One
+// pass of a small scene, time of one kernel over staged, square film at depth
+// 3, at 7, and film three times as wide as high (which sees past the box) at
+// depth 3: 2k triangles 60k paths 0.93, 1.03, 0.83, 100k 1.04, 1.27, 0.83,
+// 130k 1.15, 1.40, 0.91, 160k 1.17, 1.40, 1.00; all material types 60k 1.13,
+// 1.46, 0.86, 100k 1.40, 2.07, 0.95, 130k 1.55, 2.20, 1.08.  100k triangles,
+// us, 16k paths 456 and 507, 32k 650 and 558.  The kernel of several passes
+// has 32 registers: 8k paths 1.14-1.22 times the staged time, 20k 1.03-1.12,
+// 90k 1.00-1.52.
 inline bool staged_pays(const DeviceScene& sc, int64_t paths, bool several, bool full) {
     if (several) return paths >= 8192;
-    if (sc.accel.M >= 16384) return paths >= 24576;
-    return paths >= (full ? 32768 : 73728);
+    if (sc.accel.M >= 16384) return paths >= 32768;
+    return paths >= (full ? 131072 : 147456);
 }
 // A differentiable step, forward and replay (2k triangles, depth 6, us): 16k
 // paths 702 in one kernel each and 709 staged, 33k 789 and 767, 65k 1043 and

@@ -403,23 +403,25 @@ constexpr int64_t kWideMaxRays = int64_t(1) << 30;  // of one grid
 constexpr int kInner = 22;
 constexpr int kRefill = 6;
 
-// Rays per warp and round: 32, fewer when n does not give 32 to eight warps
-// per SM (see wide_blocks).
+// Rays per warp and round: 32, fewer when n does not give 32 to kThinWarps
+// warps per SM (see wide_blocks).
+constexpr int kThinWarps = 16;
 __host__ __device__ __forceinline__ int wide_group(int64_t n, int sms) {
-    const int64_t g = (n + (int64_t)sms * 8 - 1) / ((int64_t)sms * 8);
+    const int64_t g = (n + (int64_t)sms * kThinWarps - 1) / ((int64_t)sms * kThinWarps);
     return (int)(g < 1 ? 1 : g > 32 ? 32 : g);
 }
 // Blocks of kWideBlock threads for up to n rays (a kernel that gets a smaller
 // number from the device takes wide_group of that): one wave of resident
 // warps, and never fewer warps than wide_group counts on.  Rays
-// too few for eight warps of 32 per SM are spread thinner over eight warps per
-// SM, so that they do not wait for each other's branches (997 rays on 2048
-// triangles 76 -> 55 us, 5000 on 1M 237 -> 198 us with the whole launch).
-// Spreading over all resident warps is slower from 60,000 rays on (88 -> 101
-// us): full warps share their loads.
+// too few for 16 warps of 32 per SM are spread thinner over 16 warps per SM,
+// so that they do not wait for each other's branches (997 rays on 2048
+// triangles 76 -> 55 us, 5000 on 1M 237 -> 198 us with the whole launch, at
+// eight warps).  With 8, 16, 24 and 40 warps per SM, us: 20000 rays on 4096
+// triangles 74, 64, 72, 81, on 4M 866, 699, 651, 653; 65536 rays 95, 87, 103,
+// 124 and 1113, 1088, 1032, 1231: full warps share their loads.
 inline unsigned wide_blocks(int64_t n, int sms) {
     const int64_t warps = (int64_t)sms * kWideBlocksPerSM * (kWideBlock / 32);
-    const int64_t full = (n + 31) / 32 > (int64_t)sms * 8 ? (n + 31) / 32 : (int64_t)sms * 8;
+    const int64_t full = (n + 31) / 32 > (int64_t)sms * kThinWarps ? (n + 31) / 32 : (int64_t)sms * kThinWarps;
     int64_t used = full < warps ? full : warps;
     used = n < used ? n : used;
     return (unsigned)((used + kWideBlock / 32 - 1) / (kWideBlock / 32));
