@@ -1,0 +1,31 @@
+"""Orderings in the device and host sources that no run can be relied on to
+show: a missing memory barrier between lanes, a call on the wrong device, an
+optional allocation ahead of one that has to succeed."""
+from __future__ import annotations
+
+import re
+from pathlib import Path
+
+CSRC = Path(__file__).resolve().parents[1] / "zillumgl_gb300" / "csrc"
+
+
+def _body(name: str, head: str) -> str:
+    """The braces behind the first occurrence of `head`, comments left out."""
+    text = re.sub(r"//[^\n]*", "", (CSRC / name).read_text())
+    start = text.index("{", text.index(head))
+    depth = 0
+    for i in range(start, len(text)):
+        depth += {"{": 1, "}": -1}.get(text[i], 0)
+        if depth == 0:
+            return text[start:i + 1]
+    raise AssertionError(f"{name}: unbalanced braces behind {head}")
+
+
+def test_subtree_bins_are_read_behind_a_barrier():
+    """The lanes of a warp fill the bins with shared-memory atomics; a warp
+    reduction does not order them before other lanes' plain reads."""
+    body = _body("bvh_build_gpu.cu", "subtree_kernel(")
+    filled = max(m.end() for m in re.finditer(r"atomic\w+\(&ws\.", body))
+    read = re.search(r"=\s*ws\.(lo|hi|cnt)\[bb\]", body).start()
+    assert filled < read
+    assert "__syncwarp();" in body[filled:read]

@@ -810,6 +810,8 @@ __global__ void __launch_bounds__(kSubtreeBlock) subtree_kernel(const Seg* __res
                 }
             }
             const uint32_t wl2 = __reduce_max_sync(full, __float_as_uint(l2));
+            // the reduction orders no memory: the bins are other lanes' atomics
+            __syncwarp();
             uint32_t lk[3], hk[3], tl[3], th[3], nleftU;
             const int bb = lane & 15;
             for (int k = 0; k < 3; k++) {
