@@ -314,7 +314,10 @@ zgl_status zgl_integrator_create(zgl_scene* scene, int32_t kind, const zgl_integ
                                  zgl_integrator** out);
 
 /* Integrator::renderOnePass (NaivePath.cpp:77-105): one sample per pixel,
- * accumulated into the frame; asynchronous on `stream`. */
+ * accumulated into the frame; asynchronous on `stream`.  Passes of one
+ * integrator that share its working lists run one after the other on the
+ * device, also on different streams and in CUDA graphs; the host calls are
+ * not to be made at the same time. */
 zgl_status zgl_integrator_render_pass(zgl_integrator* integ, void* stream);
 
 /* `passes` consecutive calls of zgl_integrator_render_pass in one go: the
@@ -472,7 +475,9 @@ zgl_status zgl_diff_forward(zgl_diff* diff, float* image, void* stream);
  * radiance and the ray casts kept by the last zgl_diff_forward (bounces past
  * the kept ones, or all of them when the casts did not fit or
  * zgl_diff_set_params ran since, are traced again; the gradient is the same
- * either way up to float atomic order). */
+ * either way up to float atomic order).  Adjoints of one forward may be queued
+ * on several streams and from several threads; those that share the
+ * renderer's working lists run one after the other on the device. */
 zgl_status zgl_diff_backward(zgl_diff* diff, const float* d_image, float* d_params, void* stream);
 
 /* One inverse-rendering step of the image loss

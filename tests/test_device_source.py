@@ -29,3 +29,16 @@ def test_subtree_bins_are_read_behind_a_barrier():
     read = re.search(r"=\s*ws\.(lo|hi|cnt)\[bb\]", body).start()
     assert filled < read
     assert "__syncwarp();" in body[filled:read]
+
+
+def test_staged_calls_take_their_turn():
+    """Two calls of one handle at once would append to the same lists, beyond
+    their ends; the batched renderer's run on its own stream."""
+    for name, heads in (("render.cu", ("void staged_passes(", "void staged_light(")),
+                        ("render_diff.cu", ("zgl_status zgl_diff_forward(", "zgl_status zgl_diff_backward("))):
+        for head in heads:
+            body = _body(name, head)
+            launch = re.search(r"ZGL_CUDA\(launch_(staged|staged_light|replay)\(", body).start()
+            assert re.search(r"const StagedTurn turn\((it|d)->pool, st\);\s*$", body[:launch]), head
+        text = (CSRC / name).read_text()
+        assert len(re.findall(r"ZGL_CUDA\(launch_(?:staged|staged_light|replay)\(", text)) == len(heads)

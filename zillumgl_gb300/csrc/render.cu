@@ -101,6 +101,7 @@ void staged_passes(zgl_integrator* it, int32_t f0, int32_t n, cudaStream_t st) {
     job.n = n;
     job.counter0 = f0 - it->curSample;
     job.out = it->d_passes;
+    const StagedTurn turn(it->pool, st);
     ZGL_CUDA(launch_staged(it->pool, job, st));
     ZGL_CUDA(plain::launch_accumulate_passes(sc, it->curSample, n, it->d_passes, it->d_frame, st));
 }
@@ -119,6 +120,7 @@ void staged_light(zgl_integrator* it, uint32_t paths, bool triple, cudaStream_t 
     job.seed = (uint32_t)it->curSample * paths + (uint32_t)it->freeCounter;
     job.scale = plain::triple_scale(sc, it->blocks, 1);
     job.film = it->d_film;
+    const StagedTurn turn(it->pool, st);
     ZGL_CUDA(launch_staged_light(it->pool, job, st));
 }
 

@@ -931,6 +931,7 @@ zgl_status zgl_diff_forward(zgl_diff* d, float* image, void* stream) {
         job.hits = d->d_hits;
         job.castDepth = kCastDepth;
         job.vis = d->d_vis;
+        const StagedTurn turn(d->pool, st);
         ZGL_CUDA(launch_staged(d->pool, job, st));
     } else if (s->fullMaterials)
         diff_forward_kernel<true><<<grid, dim3(kTileX, kTileY), 0, st>>>(s->view(), path_params(d->params), tilesX,
@@ -971,6 +972,7 @@ zgl_status zgl_diff_backward(zgl_diff* d, const float* d_image, float* d_params,
         job.hits = hits;
         job.vis = vis;
         job.grad = d->d_grad;
+        const StagedTurn turn(d->pool, st);
         ZGL_CUDA(launch_replay(d->pool, s->view(), path_params(d->params), s->fullMaterials, job, d_params, st));
     } else if (s->fullMaterials)
         diff_backward_kernel<true><<<grid, dim3(kTileX, kTileY), 0, st>>>(s->view(), path_params(d->params), di,

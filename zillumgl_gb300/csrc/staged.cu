@@ -295,15 +295,39 @@ bool staged_alloc(StagedPool& pool, int64_t total) {
         }
     }
     p.paths = n;
-    staged_free(pool);
+    p.turns = pool.turns;
+    if (!p.turns) {
+        p.turns = new StagedTurns();
+        if (cudaEventCreateWithFlags(&p.turns->done, cudaEventDisableTiming) != cudaSuccess) {
+            cudaGetLastError();
+            p.turns->done = nullptr;
+            staged_free(p);
+            return false;
+        }
+    }
+    if (pool.arena) cudaFree(pool.arena);
     pool = p;
     return true;
 }
 
 void staged_free(StagedPool& p) {
     if (p.arena) cudaFree(p.arena);
-    p.arena = nullptr;
-    p.paths = 0;
+    if (p.turns) {
+        if (p.turns->done) cudaEventDestroy(p.turns->done);
+        delete p.turns;
+    }
+    p = StagedPool{};
+}
+
+StagedTurn::StagedTurn(const StagedPool& pool, cudaStream_t st) : t_(pool.turns), st_(st), lock_(pool.turns->mutex) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &status) != cudaSuccess) cudaGetLastError();  // the launches will say what is wrong
+    captured_ = status == cudaStreamCaptureStatusActive;
+    ZGL_CUDA(cudaStreamWaitEvent(st, t_->done, captured_ ? cudaEventWaitExternal : cudaEventWaitDefault));
+}
+
+StagedTurn::~StagedTurn() {
+    cudaEventRecordWithFlags(t_->done, st_, captured_ ? cudaEventRecordExternal : cudaEventRecordDefault);
 }
 
 cudaError_t launch_staged(const StagedPool& pool, const StagedJob& job, cudaStream_t st) {

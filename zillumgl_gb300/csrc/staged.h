@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <mutex>
 
 #include "device_scene.h"
 
@@ -21,10 +22,18 @@ constexpr int32_t kStagedMaxDepth = 24;
 // Sample indices whose Sobol rows fit the pool's table.
 constexpr int32_t kStagedRows = 256;
 
+// Order of the calls that share a pool: each waits on the device for the one
+// before it, whatever streams they are enqueued on.
+struct StagedTurns {
+    std::mutex mutex;  // of one call's wait, launches and record
+    cudaEvent_t done = nullptr;
+};
+
 // Device memory of a staged render of up to `paths` paths at a time.
 struct StagedPool {
     void* arena = nullptr;
     int64_t paths = 0;
+    StagedTurns* turns = nullptr;  // from the first allocation on
     float4 *org[2], *dir[2], *thr[2], *pos[2];
     uint2* rng[2];
     int2* hit;
@@ -38,6 +47,24 @@ struct StagedPool {
 // the smaller pool).
 bool staged_alloc(StagedPool& p, int64_t total);
 void staged_free(StagedPool& p);
+
+// Held while a call enqueues work on a pool (lists, counters, and whatever else
+// of its handle such calls share).  Two calls that ran at once would append to
+// the same lists, beyond their ends.  Captured calls take their turn when the
+// graph runs: the wait and the record become nodes of it.
+class StagedTurn {
+public:
+    StagedTurn(const StagedPool& pool, cudaStream_t st);
+    ~StagedTurn();
+    StagedTurn(const StagedTurn&) = delete;
+    StagedTurn& operator=(const StagedTurn&) = delete;
+
+private:
+    StagedTurns* t_;
+    cudaStream_t st_;
+    bool captured_ = false;
+    std::unique_lock<std::mutex> lock_;
+};
 
 // Samples s in [first, first + n) of every pixel of a scene, `maxDepth` at
 // most kStagedMaxDepth.  Sample s uses Sobol row sample_offset(s) and
