@@ -42,3 +42,14 @@ def test_staged_calls_take_their_turn():
             assert re.search(r"const StagedTurn turn\((it|d)->pool, st\);\s*$", body[:launch]), head
         text = (CSRC / name).read_text()
         assert len(re.findall(r"ZGL_CUDA\(launch_(?:staged|staged_light|replay)\(", text)) == len(heads)
+
+
+def test_export_runs_on_the_accelerators_device():
+    """An export allocates and launches; the current device may be another one
+    than the tree's, as in the trace calls."""
+    for entry in ("zgl_accel_export", "zgl_trace_closest", "zgl_trace_any", "zgl_trace_count",
+                  "zgl_trace_closest_noalloc"):
+        body = _body("accel.cu", f"zgl_status {entry}(")
+        guard = body.find("DeviceGuard dg(accel->device);")
+        work = re.search(r"export_device_tree\(|launch_trace_|Staging st\(|cudaMemcpy", body).start()
+        assert 0 <= guard < work, entry

@@ -737,6 +737,7 @@ zgl_status zgl_accel_export(const zgl_accel* accel, float* bounds, int32_t* hit_
     if (accel->M > 0 && (!bounds || !hit_table))
         fail(ZGL_ERR_INVALID_ARG, "zgl_accel_export: NULL output array");
     if (accel->M > 0 && accel->device_built) {
+        DeviceGuard dg(accel->device);
         export_device_tree(accel, bounds, hit_table);
     } else if (accel->M > 0) {
         std::memcpy(bounds, accel->host.bounds.data(), sizeof(float) * accel->M * 6);
