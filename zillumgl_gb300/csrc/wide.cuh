@@ -173,13 +173,16 @@ struct WidePad {
 
     __device__ __forceinline__ void set(const DeviceAccel& a, const TraceRay& r) {
         // an axis boxHit does not measure along becomes an inside test: any
-        // difference times 1e30 is below 0 or beyond every distance
+        // difference times infinity is decisive, however small, and the NaN
+        // of a zero difference is dropped by max and min (the child is then
+        // entered, a superset)
+        const float pass = __int_as_float(0x7f800000);
         px = r.mode == 4 ? r.sx : r.mode != 0;
         py = r.mode == 4 ? r.sy : r.mode != 1;
         pz = r.mode == 4 ? r.sz : r.mode != 2;
-        ix = px ? 1e30f : r.dinv.x;
-        iy = py ? 1e30f : r.dinv.y;
-        iz = pz ? 1e30f : r.dinv.z;
+        ix = px ? pass : r.dinv.x;
+        iy = py ? pass : r.dinv.y;
+        iz = pz ? pass : r.dinv.z;
         padA = padB = 0.0f;
         if (r.mode == 4) {
             const float4 rl = __ldg(a.nodes), rh = __ldg(a.nodes + 1);
