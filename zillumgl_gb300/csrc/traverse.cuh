@@ -491,6 +491,14 @@ __device__ __forceinline__ void finish_long_rays(const DeviceAccel& a, const Tra
 // over.
 constexpr int kLongRayBudget = 256;
 
+// The lane's number in its warp.  The integrators' blocks are two-dimensional
+// (16x8): threadIdx.x counts only to 15 there and comes twice in a warp.
+__device__ __forceinline__ int hw_lane() {
+    int l;
+    asm("mov.u32 %0, %%laneid;" : "=r"(l));
+    return l;
+}
+
 // traverse_warp for a group of lanes `group` (the lanes of the warp that
 // called together; a window is as wide as the group, entry k + rank on the
 // lane of that rank).  Only MODE 4 rays are handed over, so only that mode
@@ -498,7 +506,7 @@ constexpr int kLongRayBudget = 256;
 template <bool ANY>
 __device__ __forceinline__ void traverse_group(unsigned group, const DeviceAccel& a, const TraceRay& r,
                                                float& dist, int& k, int& closest) {
-    const int lane = threadIdx.x & 31;
+    const int lane = hw_lane();
     const int width = __popc(group);
     const int rank = __popc(group & ((1u << lane) - 1u));
     const float4* __restrict__ base = a.nodes + (size_t)r.face * (size_t)a.M * 2;
@@ -546,7 +554,7 @@ __device__ __forceinline__ void traverse_group(unsigned group, const DeviceAccel
 template <bool ANY>
 __device__ __forceinline__ void finish_long_rays_group(unsigned group, const DeviceAccel& a, const TraceRay& r,
                                                        float& dist, int& k, int& closest, bool done) {
-    const int lane = threadIdx.x & 31;
+    const int lane = hw_lane();
     unsigned pending = __ballot_sync(group, !done);
     while (pending) {
         const int src = __ffs(pending) - 1;
