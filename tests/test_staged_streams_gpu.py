@@ -6,7 +6,7 @@ from __future__ import annotations
 import numpy as np
 import pytest
 
-from zillumgl_gb300.scene import DiffRenderer, LightIntegrator, Scene
+from zillumgl_gb300.scene import DiffRenderer, LightIntegrator, PathIntegrator, Scene
 from zillumgl_gb300.synthetic import cornell_scene, diff_scene
 
 from tests.test_light_gpu import _check
@@ -79,3 +79,29 @@ def test_gradients_of_two_adjoints_on_two_streams(zgl_lib, cuda):
             assert float((g.double() - want[s]).abs().max()) <= 1e-5 * float(want[s].abs().max())
     r.close()
     sc.close()
+
+
+def test_captured_pass_outlives_a_larger_call(zgl_lib, cuda):
+    """Several passes at once need larger buffers; a pass captured before that
+    still runs on its own."""
+    import torch
+
+    sc = Scene(cornell_scene(seed=44, width=401, height=397))  # one pass runs staged
+    ten, it = PathIntegrator(sc, max_depth=4), PathIntegrator(sc, max_depth=4)
+    ten.render_passes(10)
+    it.render_one_pass()
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        it.render_one_pass(stream=stream)  # sample 1, in the frame when the graph runs
+    it.render_passes(8)
+    fill = [torch.full((1 << 24,), 7.0, device=cuda) for _ in range(8)]  # takes what was given back
+    graph.replay()
+    torch.cuda.synchronize()
+    assert all(bool((f == 7.0).all()) for f in fill)
+    got, want = it.get_frame()[0][..., :3], ten.get_frame()[0][..., :3]
+    # ten positive float32 terms in another order: nine roundings of 2^-24 each way
+    assert np.all(np.abs(got - want) <= 18 * 2.0 ** -24 * np.abs(want))
+    for x in (ten, it, sc):
+        x.close()

@@ -275,7 +275,7 @@ zgl_status zgl_integrator_render_passes(zgl_integrator* it, int32_t passes, void
         const zgl_scene* sc = it->scene;
         const size_t need = (size_t)3 * sc->filmW * sc->filmH * (size_t)n;
         if (need > it->passesCap) {
-            if (it->d_passes) ZGL_CUDA(cudaFree(it->d_passes));
+            staged_release(it->pool, it->d_passes);
             it->d_passes = nullptr;
             it->passesCap = 0;
             ZGL_CUDA(cudaMalloc(&it->d_passes, sizeof(float) * need));

@@ -305,15 +305,22 @@ bool staged_alloc(StagedPool& pool, int64_t total) {
             return false;
         }
     }
-    if (pool.arena) cudaFree(pool.arena);
+    staged_release(pool, pool.arena);
     pool = p;
     return true;
+}
+
+void staged_release(const StagedPool& p, void* memory) {
+    if (!memory) return;
+    if (p.turns && p.turns->captured) p.turns->retired.push_back(memory);
+    else cudaFree(memory);
 }
 
 void staged_free(StagedPool& p) {
     if (p.arena) cudaFree(p.arena);
     if (p.turns) {
         if (p.turns->done) cudaEventDestroy(p.turns->done);
+        for (void* m : p.turns->retired) cudaFree(m);
         delete p.turns;
     }
     p = StagedPool{};
@@ -323,6 +330,7 @@ StagedTurn::StagedTurn(const StagedPool& pool, cudaStream_t st) : t_(pool.turns)
     cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &status) != cudaSuccess) cudaGetLastError();  // the launches will say what is wrong
     captured_ = status == cudaStreamCaptureStatusActive;
+    t_->captured = t_->captured || captured_;
     ZGL_CUDA(cudaStreamWaitEvent(st, t_->done, captured_ ? cudaEventWaitExternal : cudaEventWaitDefault));
 }
 

@@ -8,6 +8,7 @@
 
 #include <cstdint>
 #include <mutex>
+#include <vector>
 
 #include "device_scene.h"
 
@@ -27,6 +28,8 @@ constexpr int32_t kStagedRows = 256;
 struct StagedTurns {
     std::mutex mutex;  // of one call's wait, launches and record
     cudaEvent_t done = nullptr;
+    bool captured = false;       // a graph holds addresses of the pool
+    std::vector<void*> retired;  // what such a graph may still use, freed with the pool
 };
 
 // Device memory of a staged render of up to `paths` paths at a time.
@@ -47,6 +50,9 @@ struct StagedPool {
 // the smaller pool).
 bool staged_alloc(StagedPool& p, int64_t total);
 void staged_free(StagedPool& p);
+// Gives back memory that calls on the pool use beside it: at once, or with the
+// pool if a graph may hold its address.
+void staged_release(const StagedPool& p, void* memory);
 
 // Held while a call enqueues work on a pool (lists, counters, and whatever else
 // of its handle such calls share).  Two calls that ran at once would append to
