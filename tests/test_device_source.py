@@ -53,3 +53,16 @@ def test_export_runs_on_the_accelerators_device():
         guard = body.find("DeviceGuard dg(accel->device);")
         work = re.search(r"export_device_tree\(|launch_trace_|Staging st\(|cudaMemcpy", body).start()
         assert 0 <= guard < work, entry
+
+
+def test_optional_memory_comes_last():
+    """The staged renderers run without their pool: it is taken behind all that
+    a handle cannot do without, and given back where that is short."""
+    for name, entry in (("render_diff.cu", "zgl_diff_create"), ("render_batch.cu", "zgl_batch_create")):
+        body = _body(name, f"zgl_status {entry}(")
+        needed = max(m.start() for m in re.finditer(r"ZGL_CUDA\(cudaMalloc\(|ZGL_CUDA\(cudaEventCreate", body))
+        assert needed < body.index("staged_alloc("), entry
+    for name, entry, array in (("render_diff.cu", "zgl_diff_step_l2", "d_dimage"),
+                               ("render.cu", "zgl_integrator_render_passes", "d_passes")):
+        body = _body(name, f"zgl_status {entry}(")
+        assert re.search(rf"staged_malloc_beside\(\w+->pool, \(void\*\*\)&\w+->{array}", body), entry

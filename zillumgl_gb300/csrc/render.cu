@@ -278,7 +278,7 @@ zgl_status zgl_integrator_render_passes(zgl_integrator* it, int32_t passes, void
             staged_release(it->pool, it->d_passes);
             it->d_passes = nullptr;
             it->passesCap = 0;
-            ZGL_CUDA(cudaMalloc(&it->d_passes, sizeof(float) * need));
+            ZGL_CUDA(staged_malloc_beside(it->pool, (void**)&it->d_passes, sizeof(float) * need));
             it->passesCap = need;
         }
         const int64_t paths = std::min(staged_paths(sc->filmW, sc->filmH, n), kStagedPaths);

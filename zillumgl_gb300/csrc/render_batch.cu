@@ -694,13 +694,6 @@ zgl_status zgl_batch_create(const zgl_render_request* requests, int32_t n, const
             q.scratch = b->d_scratch + off;
             off += (size_t)std::min(b->chunkLen, q.spp) * (size_t)q.npix * 3;
         }
-        // the staged path tracer's pool, for the largest request of a launch
-        int64_t paths = 0;
-        for (const auto& q : b->req) {
-            const int n = std::min(b->chunkLen, q.spp);
-            if (runs_staged(q, n)) paths = std::max(paths, staged_paths(q.sc.filmW, q.sc.filmH, n));
-        }
-        if (paths > 0) staged_alloc(b->pool, paths);
         const int nChunks = (b->maxSpp + b->chunkLen - 1) / b->chunkLen;
         b->nchunks_cap = nChunks * ((n + kMaxReqPerLaunch - 1) / kMaxReqPerLaunch);
         ZGL_CUDA(cudaMalloc(&b->d_counters, sizeof(unsigned long long) * (size_t)b->nchunks_cap));
@@ -708,6 +701,14 @@ zgl_status zgl_batch_create(const zgl_render_request* requests, int32_t n, const
         ZGL_CUDA(cudaEventCreateWithFlags(&b->ev_in, cudaEventDisableTiming));
         ZGL_CUDA(cudaEventCreateWithFlags(&b->ev_out, cudaEventDisableTiming));
         b->cfg = resolve(cfg);
+        // the staged path tracer's pool, for the largest request of a launch;
+        // last, so that it takes no memory from what has to be there
+        int64_t paths = 0;
+        for (const auto& q : b->req) {
+            const int n = std::min(b->chunkLen, q.spp);
+            if (runs_staged(q, n)) paths = std::max(paths, staged_paths(q.sc.filmW, q.sc.filmH, n));
+        }
+        if (paths > 0) staged_alloc(b->pool, paths);
     } catch (...) {
         batch_free(b);
         throw;

@@ -839,8 +839,6 @@ zgl_status zgl_diff_create(zgl_scene* scene, const zgl_integrator_params* params
             ZGL_CUDA(cudaMalloc(&d->d_hits, sizeof(int2) * kCastDepth * paths));
             ZGL_CUDA(cudaMalloc(&d->d_vis, sizeof(uint32_t) * paths));
         }
-        if (staged_covers(scene->view(), d->params.max_depth) && staged_diff_pays((int64_t)paths))
-            staged_alloc(d->pool, staged_paths(scene->filmW, scene->filmH, spp));
         std::vector<int32_t> inst((size_t)std::max(scene->nLight, 1), 0);
         for (int k = 0; k < d->ninst; k++)
             for (uint32_t t = d->lightFirst[(size_t)k]; t < d->lightFirst[(size_t)k + 1]; t++) inst[t] = k;
@@ -854,9 +852,17 @@ zgl_status zgl_diff_create(zgl_scene* scene, const zgl_integrator_params* params
             std::memcpy(&d->params_host[(size_t)kDiffMatParams * m], v, sizeof(v));
         }
         for (int k = 0; k < 3 * d->ninst; k++) d->params_host[(size_t)kDiffMatParams * d->nmat + k] = d->instPower[(size_t)k];
-        if (d->pool.arena) ZGL_CUDA(cudaMalloc(&d->d_grad, sizeof(double) * (size_t)std::max(d->nparams, 1)));
         ZGL_CUDA(cudaMalloc(&d->d_values, sizeof(float) * (size_t)std::max(d->nparams, 1)));
         ZGL_CUDA(cudaMemcpy(d->d_values, d->params_host.data(), sizeof(float) * (size_t)d->nparams, cudaMemcpyHostToDevice));
+        // last, so that it takes no memory from what has to be there; without
+        // it the one-kernel forward and replay run
+        if (staged_covers(scene->view(), d->params.max_depth) && staged_diff_pays((int64_t)paths) &&
+            staged_alloc(d->pool, staged_paths(scene->filmW, scene->filmH, spp)) &&
+            cudaMalloc(&d->d_grad, sizeof(double) * (size_t)std::max(d->nparams, 1)) != cudaSuccess) {
+            cudaGetLastError();
+            d->d_grad = nullptr;
+            staged_free(d->pool);
+        }
     } catch (...) {
         if (d->d_samples) cudaFree(d->d_samples);
         if (d->d_hits) cudaFree(d->d_hits);
@@ -997,7 +1003,7 @@ zgl_status zgl_diff_step_l2(zgl_diff* d, const float* target, float loss_scale, 
     const zgl_scene* s = d->scene;
     cudaStream_t st = (cudaStream_t)stream;
     const int64_t n = (int64_t)s->filmW * s->filmH * 3;
-    if (!d->d_dimage) ZGL_CUDA(cudaMalloc(&d->d_dimage, sizeof(float) * (size_t)n));
+    if (!d->d_dimage) ZGL_CUDA(staged_malloc_beside(d->pool, (void**)&d->d_dimage, sizeof(float) * (size_t)n));
     zgl_status r = zgl_diff_forward(d, image, stream);
     if (r != ZGL_OK) return r;
     ZGL_CUDA(cudaMemsetAsync(loss, 0, sizeof(float), st));

@@ -316,6 +316,16 @@ void staged_release(const StagedPool& p, void* memory) {
     else cudaFree(memory);
 }
 
+cudaError_t staged_malloc_beside(StagedPool& p, void** memory, size_t bytes) {
+    cudaError_t e = cudaMalloc(memory, bytes);
+    if (e != cudaErrorMemoryAllocation || !p.arena) return e;
+    cudaGetLastError();
+    staged_release(p, p.arena);
+    p.arena = nullptr;
+    p.paths = 0;
+    return cudaMalloc(memory, bytes);
+}
+
 void staged_free(StagedPool& p) {
     if (p.arena) cudaFree(p.arena);
     if (p.turns) {

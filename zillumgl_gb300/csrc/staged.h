@@ -53,6 +53,9 @@ void staged_free(StagedPool& p);
 // Gives back memory that calls on the pool use beside it: at once, or with the
 // pool if a graph may hold its address.
 void staged_release(const StagedPool& p, void* memory);
+// cudaMalloc of memory that the handle needs whether or not it runs staged:
+// gives the pool back where there is not enough beside it.
+cudaError_t staged_malloc_beside(StagedPool& p, void** memory, size_t bytes);
 
 // Held while a call enqueues work on a pool (lists, counters, and whatever else
 // of its handle such calls share).  Two calls that ran at once would append to
