@@ -66,3 +66,9 @@ def test_optional_memory_comes_last():
                                ("render.cu", "zgl_integrator_render_passes", "d_passes")):
         body = _body(name, f"zgl_status {entry}(")
         assert re.search(rf"staged_malloc_beside\(\w+->pool, \(void\*\*\)&\w+->{array}", body), entry
+
+
+def test_export_needs_no_device_memory():
+    """An export without memory to spare rearranges the records on the host."""
+    body = _body("wide_build.cu", "void export_device_tree(")
+    assert "ZGL_ERR_OOM" not in body and "return export_on_host(" in body[body.index("cudaMalloc("):]
