@@ -429,7 +429,8 @@ zgl_status zgl_batch_render(zgl_batch* batch, void* stream);
 
 /* Times the flat schedule and every combination of block size, queue
  * capacity and regeneration threshold of the persistent one on the first
- * samples of the batch, keeps the fastest for later renders and returns it
+ * samples of the batch (two of a request, more of a small film where the
+ * flat schedule needs them to take the route of the whole render), keeps the fastest for later renders and returns it
  * in `chosen` (may be NULL).  Overwrites the frames. */
 zgl_status zgl_batch_autotune(zgl_batch* batch, void* stream, zgl_batch_config* chosen);
 

@@ -442,7 +442,7 @@ struct zgl_batch {
     uint32_t* d_rows = nullptr;     // maxSpp x 256 Sobol values
     float* d_scratch = nullptr;     // per request: min(spp, chunkLen) x npix x 3
     unsigned long long* d_counters = nullptr;
-    zgl::StagedPool pool;           // the flat schedule's, when every request runs staged
+    zgl::StagedPool pool;           // the flat schedule's, for the requests that run staged
     int32_t nchunks_cap = 0;
     zgl_batch_config cfg{};
     cudaStream_t stream = nullptr;
@@ -493,25 +493,36 @@ bool runs_staged(const BatchRequest& q, int n) {
     return staged_covers(q.sc, q.pp.maxDepth) && staged_pays_in_batch(q.sc, (int64_t)q.npix * n);
 }
 
+// Samples of a request that a trial of the autotuner renders: two, or as many
+// as it takes for the route (staged or shared) that the render takes.
+int trial_samples(const zgl_batch* b, const BatchRequest& q) {
+    int n = std::min(2, q.spp);
+    if (b->pool.arena && runs_staged(q, std::min(b->chunkLen, q.spp)))
+        while (!runs_staged(q, n)) n++;
+    return n;
+}
+
 // Enqueues the whole render on `st`: frame clears, then per chunk of sample
 // indices one persistent launch per group of up to 64 requests that need
 // samples of the chunk (each with its own counter reset) and the in-order
-// frame updates of that group.  `first_samples` > 0 renders only that many
-// sample indices (autotuning).
-void enqueue_render(zgl_batch* b, const zgl_batch_config& c, cudaStream_t st, int first_samples) {
+// frame updates of that group.  `trial` renders only the first samples
+// (autotuning).
+void enqueue_render(zgl_batch* b, const zgl_batch_config& c, cudaStream_t st, bool trial) {
     for (const auto& r : b->req)
         ZGL_CUDA(cudaMemsetAsync(r.frame, 0, sizeof(float4) * (size_t)r.npix, st));
-    const int nsamples = first_samples > 0 ? std::min(first_samples, b->maxSpp) : b->maxSpp;
+    std::vector<int> samples;
+    for (const auto& r : b->req) samples.push_back(trial ? trial_samples(b, r) : r.spp);
+    const int nsamples = *std::max_element(samples.begin(), samples.end());
     int k = 0;
     for (int j0 = 0; j0 < nsamples; j0 += b->chunkLen) {
         const int j1 = std::min(j0 + b->chunkLen, nsamples);
         std::vector<int> active;
         for (int i = 0; i < b->nreq; i++)
-            if (b->req[(size_t)i].spp > j0) active.push_back(i);
+            if (samples[(size_t)i] > j0) active.push_back(i);
         // largest work first, so that small requests fill the launch's tail
         auto work = [&](int i) {
             const BatchRequest& q = b->req[(size_t)i];
-            return (double)q.npix * (double)(std::min(j1, q.spp) - j0) * (double)std::max(q.pp.maxDepth, 1);
+            return (double)q.npix * (double)(std::min(j1, samples[(size_t)i]) - j0) * (double)std::max(q.pp.maxDepth, 1);
         };
         std::stable_sort(active.begin(), active.end(), [&](int x, int y) { return work(x) > work(y); });
         for (size_t g0 = 0; g0 < active.size(); g0 += kMaxReqPerLaunch) {
@@ -521,7 +532,7 @@ void enqueue_render(zgl_batch* b, const zgl_batch_config& c, cudaStream_t st, in
             int64_t base = 0, pbase = 0;
             for (size_t j = g0; j < active.size() && (int)(j - g0) < kMaxReqPerLaunch; j++) {
                 BatchRequest q = b->req[(size_t)active[j]];
-                q.j1 = std::min(j1, q.spp);
+                q.j1 = std::min(j1, samples[(size_t)active[j]]);
                 q.itemBase = base;
                 base += (int64_t)(q.j1 - j0) * q.perSample;
                 L.req[L.nreq++] = q;
@@ -745,7 +756,7 @@ zgl_status zgl_batch_render(zgl_batch* b, void* stream) {
         cudaGraph_t graph = nullptr;
         ZGL_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
         try {
-            enqueue_render(b, b->cfg, b->stream, 0);
+            enqueue_render(b, b->cfg, b->stream, false);
         } catch (...) {
             cudaGraph_t g = nullptr;
             cudaStreamEndCapture(b->stream, &g);
@@ -784,7 +795,7 @@ zgl_status zgl_batch_autotune(zgl_batch* b, void* stream, zgl_batch_config* chos
     float bestMs = 1e30f;
     auto trial = [&](const zgl_batch_config& c) {
         ZGL_CUDA(cudaEventRecord(e0, st));
-        enqueue_render(b, c, st, 2);
+        enqueue_render(b, c, st, true);
         ZGL_CUDA(cudaEventRecord(e1, st));
         ZGL_CUDA(cudaEventSynchronize(e1));
         float ms = 0.0f;
