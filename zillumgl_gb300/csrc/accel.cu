@@ -533,7 +533,8 @@ zgl_accel* accel_create(const float* vertices, const uint32_t* indices, int64_t 
         ZGL_CUDA(cudaGetDevice(&a->device));
         ZGL_CUDA(cudaMalloc(&a->d_counter, 256));
         a->ntri = ntri;
-        build_bvh(vertices, indices, a->ntri, a->host, host_threads());
+        HostWords words;
+        build_bvh(vertices, indices, a->ntri, a->host, host_threads(), &words);
         a->M = a->host.M;
         if (a->M > 0) {
             size_t nb = sizeof(float) * a->M * 6, nh = sizeof(int32_t) * a->M * 18;
@@ -560,16 +561,18 @@ zgl_accel* accel_create(const float* vertices, const uint32_t* indices, int64_t 
             }
             ZGL_CUDA(cudaMemcpy(a->d_tris, tris.data(), sizeof(float4) * tris.size(), cudaMemcpyHostToDevice));
             if (a->ntri > 1) {
-                std::vector<float4> dfs((size_t)a->M * 2);
-                std::vector<float> l2((size_t)a->M);
-                host_dfs(a->host, dfs.data(), l2.data());
-                DevicePtr<float> d_l2(l2.size());
-                ZGL_CUDA(cudaMalloc(&a->d_dfs, sizeof(float4) * dfs.size()));
-                ZGL_CUDA(cudaMemcpy(a->d_dfs, dfs.data(), sizeof(float4) * dfs.size(), cudaMemcpyHostToDevice));
-                ZGL_CUDA(cudaMemcpy(d_l2.p, l2.data(), sizeof(float) * l2.size(), cudaMemcpyHostToDevice));
+                const size_t M = (size_t)a->M, word = sizeof(uint32_t) * M;
+                DevicePtr<uint32_t> w(3 * M);  // sizeIndices, leaves, l2
+                ZGL_CUDA(cudaMemcpy(w.p, a->host.sizeIndices.data(), word, cudaMemcpyHostToDevice));
+                ZGL_CUDA(cudaMemcpy(w.p + M, words.leaves.get(), word, cudaMemcpyHostToDevice));
+                ZGL_CUDA(cudaMemcpy(w.p + 2 * M, words.l2.get(), word, cudaMemcpyHostToDevice));
+                const auto* sizes = reinterpret_cast<const int32_t*>(w.p);
+                const auto* l2 = reinterpret_cast<const float*>(w.p + 2 * M);
+                ZGL_CUDA(cudaMalloc(&a->d_dfs, sizeof(float4) * 2 * a->M));
+                ZGL_CUDA(launch_dfs_records(d_bounds, sizes, w.p + M, a->M, a->d_dfs, 0));
                 ZGL_CUDA(cudaMalloc(&a->d_wide, sizeof(float4) * 4 * (a->ntri - 1)));
                 ZGL_CUDA(cudaMalloc(&a->d_wtris, sizeof(float4) * 4 * a->ntri));
-                build_wide(a, d_l2.p, nullptr, 0);
+                build_wide(a, l2, nullptr, 0);
                 ZGL_CUDA(cudaDeviceSynchronize());
             }
             ZGL_CUDA(cudaDeviceSynchronize());

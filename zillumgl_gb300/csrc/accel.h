@@ -139,8 +139,9 @@ void build_bvh_device(const float* v, int64_t nv, const uint32_t* idx, int small
 // and d_wtris, unless the device word `err` (may be null) is set.
 // Asynchronous on `s`.
 void build_wide(zgl_accel* a, const float* l2, const uint32_t* err, cudaStream_t s);
-// dfs nodes and l2 of a host-built tree, as float4[M*2] and float[M].
-void host_dfs(const HostBVH& h, float4* dfs, float* l2);
+// dfs nodes of a host-built tree from its bounds, sizeIndices and HostWords.
+cudaError_t launch_dfs_records(const float* bounds, const int32_t* sizes, const uint32_t* leaves, int64_t M,
+                               float4* dfs, cudaStream_t s);
 // PackedBVH of a device-built tree into host memory: bounds float[M*6], hit
 // table int32[6*M*3].
 void export_device_tree(const zgl_accel* a, float* bounds, int32_t* hit_table);

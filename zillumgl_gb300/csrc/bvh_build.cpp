@@ -14,6 +14,7 @@
 #include <atomic>
 #include <condition_variable>
 #include <cstring>
+#include <exception>
 #include <mutex>
 #include <thread>
 
@@ -259,19 +260,43 @@ void hit_table_face(const float* bounds, const int32_t* sizeIndices, int64_t M, 
     (void)M;
 }
 
+// HostWords of a finished tree: leaves and depths from the front, diagonals
+// from the back.
+void fill_words(const float* bounds, const int32_t* sizeIndices, int64_t M, uint32_t* words, float* l2) {
+    std::vector<int64_t> ends;  // ends of the open ancestors' subtrees
+    uint32_t leaves = 0;
+    for (int64_t k = 0; k < M; k++) {
+        while (!ends.empty() && ends.back() <= k) ends.pop_back();
+        words[k] = leaves | (uint32_t)(ends.size() & 1u) << 31;
+        if (sizeIndices[k] & kLeafMask) leaves++;
+        else ends.push_back(k + sizeIndices[k]);
+    }
+    for (int64_t k = M - 1; k >= 0; k--) {
+        if (sizeIndices[k] & kLeafMask) {  // a leaf's bounds are its triangle's box
+            const float* b = bounds + 6 * k;
+            const float x = b[3] - b[0], y = b[4] - b[1], z = b[5] - b[2];
+            l2[k] = x * x + y * y + z * z;
+        } else {
+            const int32_t l = sizeIndices[k + 1];
+            l2[k] = std::max(l2[k + 1], l2[k + 1 + ((l & kLeafMask) ? 1 : l)]);
+        }
+    }
+}
+
 }  // namespace
 
-void build_bvh(const float* v, const uint32_t* idx, int64_t ntri, HostBVH& out, int nthreads) {
+void build_bvh(const float* v, const uint32_t* idx, int64_t ntri, HostBVH& out, int nthreads, HostWords* words) {
     out.ntri = ntri;
     out.M = ntri > 0 ? 2 * ntri - 1 : 0;
     out.bounds.resize((size_t)out.M * 6);
     out.sizeIndices.resize((size_t)out.M);
     out.hitTable.resize((size_t)out.M * 18);
-    build_bvh_into(v, idx, ntri, out.bounds.data(), out.sizeIndices.data(), out.hitTable.data(), nthreads);
+    build_bvh_into(v, idx, ntri, out.bounds.data(), out.sizeIndices.data(), out.hitTable.data(), nthreads,
+                   words);
 }
 
 void build_bvh_into(const float* v, const uint32_t* idx, int64_t ntri, float* bounds, int32_t* sizeIndices,
-                    int32_t* hitTable, int nthreads) {
+                    int32_t* hitTable, int nthreads, HostWords* words) {
     if (ntri <= 0) return;
     const int64_t M = 2 * ntri - 1;
     if (nthreads < 1) nthreads = 1;
@@ -304,10 +329,23 @@ void build_bvh_into(const float* v, const uint32_t* idx, int64_t ntri, float* bo
     for (int t = 0; t < nthreads; t++) th.emplace_back([&b] { b.worker(); });
     for (auto& x : th) x.join();
 
+    if (words) {
+        words->leaves.reset(new uint32_t[(size_t)M]);
+        words->l2.reset(new float[(size_t)M]);
+    }
     std::vector<std::thread> faces;
     for (int f = 0; f < 6; f++)
         faces.emplace_back([=] { hit_table_face(bounds, sizeIndices, M, f, hitTable + (size_t)M * 3 * f); });
+    std::exception_ptr error;
+    if (words) {  // beside the tables, which take longer
+        try {
+            fill_words(bounds, sizeIndices, M, words->leaves.get(), words->l2.get());
+        } catch (...) {
+            error = std::current_exception();
+        }
+    }
     for (auto& x : faces) x.join();
+    if (error) std::rethrow_exception(error);
 }
 
 }  // namespace zgl

@@ -136,6 +136,16 @@ wide_kernel(const float4* __restrict__ dfs, const float* __restrict__ l2, int64_
     o[3] = make_uint4(plane[4], plane[5], swaps, 0u);
 }
 
+// DFS records of a host-built tree.
+__global__ void dfs_records_kernel(const float* __restrict__ bounds, const int32_t* __restrict__ sizes,
+                                   const uint32_t* __restrict__ leaves, int64_t M, float4* __restrict__ dfs) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= M) return;
+    const float* b = bounds + 6 * i;
+    dfs[2 * i] = make_float4(b[0], b[1], b[2], __int_as_float(sizes[i]));
+    dfs[2 * i + 1] = make_float4(b[3], b[4], b[5], __uint_as_float(leaves[i]));
+}
+
 __global__ void bounds_kernel(const float4* __restrict__ dfs, int64_t first, int64_t n, float* __restrict__ out) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -172,35 +182,10 @@ void build_wide(zgl_accel* a, const float* l2, const uint32_t* err, cudaStream_t
     ZGL_CUDA(cudaGetLastError());
 }
 
-void host_dfs(const HostBVH& h, float4* dfs, float* l2) {
-    auto bits = [](uint32_t u) {
-        float f;
-        std::memcpy(&f, &u, 4);
-        return f;
-    };
-    std::vector<int64_t> ends;  // ends of the open ancestors' subtrees
-    uint32_t leaves = 0;
-    for (int64_t k = 0; k < h.M; k++) {
-        while (!ends.empty() && ends.back() <= k) ends.pop_back();
-        const float* b = h.bounds.data() + 6 * k;
-        const uint32_t w0 = (uint32_t)h.sizeIndices[k];
-        const uint32_t odd = (uint32_t)(ends.size() & 1u);
-        dfs[2 * k] = make_float4(b[0], b[1], b[2], bits(w0));
-        dfs[2 * k + 1] = make_float4(b[3], b[4], b[5], bits(leaves | odd << 31));
-        if (w0 & kTop) leaves++;
-        else ends.push_back(k + (int64_t)w0);
-    }
-    for (int64_t k = h.M - 1; k >= 0; k--) {
-        const uint32_t w0 = (uint32_t)h.sizeIndices[k];
-        if (w0 & kTop) {  // a leaf's bounds are its triangle's box
-            const float* b = h.bounds.data() + 6 * k;
-            const float x = b[3] - b[0], y = b[4] - b[1], z = b[5] - b[2];
-            l2[k] = x * x + y * y + z * z;
-        } else {
-            const uint32_t l = (uint32_t)h.sizeIndices[k + 1];
-            l2[k] = std::max(l2[k + 1], l2[k + 1 + ((l & kTop) ? 1 : (int64_t)l)]);
-        }
-    }
+cudaError_t launch_dfs_records(const float* bounds, const int32_t* sizes, const uint32_t* leaves, int64_t M,
+                               float4* dfs, cudaStream_t s) {
+    dfs_records_kernel<<<(unsigned)((M + 255) / 256), 256, 0, s>>>(bounds, sizes, leaves, M, dfs);
+    return cudaGetLastError();
 }
 
 namespace {
