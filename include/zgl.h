@@ -109,8 +109,11 @@ zgl_status zgl_bvh_build_host(const float* vertices, size_t n_vertices,
  *     reference's visiting order, resident warps whose lanes take the next
  *     ray as theirs ends; a ray with a direction component below 1e-6 in
  *     magnitude (boxHit's near-zero branch can make it visit tens of
- *     thousands of table entries) that outruns its budget is finished on the
- *     threaded table by its whole warp, 32 consecutive entries at a time.
+ *     thousands of table entries) that outruns its budget of nodes is
+ *     finished on the threaded table by its whole warp, 128 consecutive
+ *     entries at a time.  Until the call's work has ended its output arrays
+ *     may hold marks for such rays (hit_id -2, occluded 2), which the kernel
+ *     reads back: they have to be readable memory of the call's own.
  *   ZGL_TRACE_THREAD_PER_RAY (1): one thread per ray, every ray on its own
  *     lane to the end (the reference's schedule).
  *   ZGL_TRACE_PERSISTENT (2): persistent warps that refill idle lanes by

@@ -14,8 +14,8 @@
 
 namespace zgl {
 
-// Paths in flight at most: two float4 x 4 + uint2 states, a hit and a shadow
-// ray each (about 230 B), 480 MB in all; a 1080p pass fits.
+// Paths in flight at most: two states of float4 x 4 + uint2, a hit and a shadow
+// ray each (200 B), 420 MB in all; a 1080p pass fits.
 constexpr int64_t kStagedPaths = 1 << 21;
 // Depth from which the one-kernel path tracer runs instead: the staged one
 // launches two kernels per bounce whether or not a path gets there.

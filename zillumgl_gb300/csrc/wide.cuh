@@ -61,7 +61,11 @@ constexpr int kWideStack = 64;            // entries per thread (local memory)
 constexpr int kWideDone = (int)0x80000000;  // bottom of the stack
 // Nodes a ray of the rarer modes visits on its lane before its warp takes it
 // over on the face table: on meshes of small triangles, where P binds, such a
-// ray needs a few hundred; with large ones, tens of thousands.
+// ray needs a few hundred; with large ones, tens of thousands.  1M camera rays
+// with a column of 1100 such rays, 1M triangles: 6.4 ms at 256 nodes, 0.99,
+// 0.99, 0.98 at 1024, 4096, 16384; 16M shadow rays 12.8, 6.42, 6.36, 6.39.
+// Trees whose root says that P cannot bind everywhere (a triangle with a
+// squared box diagonal of 0.7 or more) get kLongRayBudget.
 constexpr int kPadBudget = 4096;
 
 // Result of one wide traversal: `ok` false when the stack ran out or a ray of
