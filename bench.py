@@ -254,7 +254,7 @@ def run_ours(args):
     out_t = torch.empty(nray, dtype=torch.float32, device=dev)
     out_occ = torch.empty(nray, dtype=torch.uint8, device=dev)
 
-    # algorithmic bytes: 32 B per table entry visited, 36 B per triangle test,
+    # the reference's walk: 32 B per table entry visited, 36 B per triangle test,
     # 24 B ray in, 8 B hit out (closest) / 4 B tmax in + 1 B flag out (any)
     for sp in specs:
         vis, tst = sp["acc"].trace_count(sp["o"], sp["d"], sp["tmax"], any_hit=sp["query"] == "any", stream=stream)
@@ -322,42 +322,55 @@ def run_ours(args):
     t_any = sum(statistics.mean(per_launch[sp["name"]]) for sp in anyq)
     dom = closest if t_closest >= t_any else anyq
     dom_ms = sum(statistics.mean(per_launch[sp["name"]]) for sp in dom) / len(dom)
-    dom_bytes = sum(sp["bytes"] for sp in dom) / len(dom)
+    # what a launch cannot do without: rays in, hits out, the mesh once
+    io = (24 + 8) if dom is closest else (24 + 4 + 1)
+    dom_bytes = io * nray + sum(36 * sp["N"] for sp in dom) / len(dom)
     achieved = dom_bytes / (dom_ms * 1e-3) / 1e9
     peak, peak_kind = measured_peaks()
-    traffic = profiled_traffic() if args.schedule == "auto" and dom is closest and len(dom) == 6 and side == 4096 else None
-    bytes_note = "32 B per table entry visited, 36 B per triangle test, ray and hit"
+    auto = args.schedule == "auto"
+    traffic = profiled_traffic() if auto and dom is closest and len(dom) == 6 and side == 4096 else None
+    # what its loads ask for, mostly of L1: the profile's count for the wide
+    # tree, the visits of the threaded tables for the other schedules
+    loaded = loaded_note = None
     if traffic:
-        # the wide tree reads fewer bytes than the table entries of the reference's walk
-        dom_bytes = traffic["load_bytes_per_launch"] + 8 * nray
-        achieved = dom_bytes / (dom_ms * 1e-3) / 1e9
-        bytes_note = traffic["load_note"]
+        loaded, loaded_note = traffic["load_bytes_per_launch"], traffic["load_note"]
+    elif not auto:
+        loaded = sum(sp["bytes"] for sp in dom) / len(dom)
+        loaded_note = "32 B per table entry visited, 36 B per triangle test, ray and hit"
+    dram = traffic["dram_bytes_per_launch"] if traffic else None
     l2, l2_sweep = l2_peak(stream)
     kname = KERNELS[resolved_schedule(args.schedule)]["closest" if dom is closest else "any"]
+
+    def gbs(b):
+        return None if b is None else round(b / (dom_ms * 1e-3) / 1e9, 1)
+
     roofline = {"bound": "latency",
-                "bound_note": "node and triangle bytes against the L2 / HBM roofline; the measured limiter is the "
-                              "instruction rate at the lanes active, L1's gather rate and dependent-load latency, not "
-                              "DRAM bandwidth: DRAM traffic is a few percent of the bytes loaded, which L1 and L2 "
-                              "serve",
-                "kernel": kname, "l2_frac": round(achieved / l2, 4), "l2_peak": round(l2, 1),
-                "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s", "frac": round(achieved / peak, 4),
-                "peak_source": f"{peak_kind} hbm_gbs (copy bandwidth)",
+                "bound_note": "the measured limiter is the instruction rate at the lanes active, L1's gather rate and "
+                              "dependent-load latency, not DRAM or L2 bandwidth",
+                "kernel": kname, "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
+                "frac": round(achieved / peak, 4), "peak_source": f"{peak_kind} hbm_gbs (copy bandwidth)",
+                "algorithmic_bytes_per_launch": int(dom_bytes),
+                "algorithmic_bytes_note": f"rays in and hits out once ({io} B a ray) and the mesh once (36 B a "
+                                          "triangle), mean over the kernel's launches of a step",
+                "traffic": dram, "traffic_gbs": gbs(dram),
+                "traffic_frac": round(dram / (dom_ms * 1e-3) / 1e9 / peak, 4) if dram else None,
+                "traffic_note": traffic.get("note") if traffic else "no ncu capture for this schedule or size",
+                "loaded_bytes_per_launch": int(loaded) if loaded else None, "loaded_gbs": gbs(loaded),
+                "loaded_note": loaded_note,
+                "l2_frac": round(loaded / (dom_ms * 1e-3) / 1e9 / l2, 4) if loaded else None,
+                "l2_note": "bytes loaded over the L2 read peak; L1 serves most of them, so L2 is busy with less",
+                "l2_peak": round(l2, 1),
                 "l2_peak_source": "zgl_measure_l2_read: L2-resident buffer read by all SMs with 16-byte ld.global.cg, "
                                   f"best of {l2_sweep} GB/s",
-                "traffic": traffic.get("dram_bytes_per_launch") if traffic else None,
-                "traffic_note": traffic.get("note") if traffic else "no ncu capture committed yet",
                 "lanes_active_per_inst": traffic.get("lanes_active_per_inst") if traffic else None,
                 "lanes_note": traffic.get("lanes_note") if traffic else None,
-                "algorithmic_bytes_per_launch": int(dom_bytes), "algorithmic_bytes_note": bytes_note,
                 "avg_launch_ms": round(dom_ms, 4)}
 
     workloads = []
     for sp in specs:
         ms = statistics.mean(per_launch[sp["name"]])
         workloads.append({"name": sp["name"], "ms": round(ms, 4), "mrays_s": round(nray / (ms * 1e-3) / 1e6, 1),
-                          "visits_per_ray": round(sp["V"] / nray, 2), "tests_per_ray": round(sp["T"] / nray, 3),
-                          "gbs": round(sp["bytes"] / (ms * 1e-3) / 1e9, 1),
-                          "l2_frac": round(sp["bytes"] / (ms * 1e-3) / 1e9 / l2, 4)})
+                          "visits_per_ray": round(sp["V"] / nray, 2), "tests_per_ray": round(sp["T"] / nray, 3)})
 
     # end to end through the C ABI with pinned host arrays
     e2e = None
